@@ -120,8 +120,9 @@ int  mdp_noise_plan(mdp_context *ctx, mdp_noise *N, int fp32, int *log2_cta_poin
  * "auto" (the autotuner's choice), "model" (the cost model's choice, nothing
  * timed), "fft:N" (the cost model's choice among one-kernel tiles of N real
  * samples), "log2_cta_points,cluster,threads" (one-kernel tiles),
- * "s,log_m1,log_m2" (three-kernel split tiles) or "c,C" (cluster four-step
- * tiles of C CTAs).  For tests and tuning; MDP_EINVAL when the plan does not
+ * "s,log_m1,log_m2" (three-kernel split tiles), "c,C" (cluster four-step
+ * tiles of C CTAs) or "r,log_m1,log_m2" (right-angle tiles: log_m1 0 and log_m2
+ * 9..12, or log_m1 1..4 and log_m2 12).  For tests and tuning; MDP_EINVAL when the plan does not
  * hold the band. */
 int  mdp_noise_set_plan(mdp_context *ctx, mdp_noise *N, int fp32, const char *plan);
 /* No counterpart in the reference.  out = N^-1 in like mdp_stbmm, but the call

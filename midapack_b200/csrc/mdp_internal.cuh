@@ -160,9 +160,10 @@ struct mdp_pointing {
 struct mdp_tile_plan {
     int     ready = 0;
     int     split = 0;     // 0: one kernel (one CTA or cluster per tile); 1: three-kernel four-step FFT;
-                           // 2: cluster four-step (ninv4.cu: C = cluster CTAs, M = 2C x 4096 points)
+                           // 2: cluster four-step (ninv4.cu: C = cluster CTAs, M = 2C x 4096 points);
+                           // 3: right-angle tiles (rtile.cu, M = 2^log_m1 x 2^log_m2 points)
     int     log_m1 = 0, log_m2 = 0;  // split: M = 2^log_m1 * 2^log_m2 complex points per tile
-    DevBuf  scratch;       // split: [n_tiles][M] complex work array
+    DevBuf  scratch;       // split: [n_tiles][M] complex work array; right-angle tiles: one launch group's
     DevBuf  ltw2, wa, wb;  // split: row-pass twiddles, W_M factor tables
     int     log2_ml = 0;   // per-CTA complex points = 2^log2_ml
     int     cluster = 1;   // CTAs per tile
@@ -265,6 +266,13 @@ template <typename T>
 int ninv4_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra);
 template <typename T>
 int ninv4_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, const T *d_in, T *d_out,
+                 const double *d_means, int ncols, int64_t col_stride, const int *d_active);
+// right-angle tiles of N^-1 (rtile.cu): whether a shape exists, tables and spectra of a plan, launch
+bool rtile_shape(int log_m1, int log_m2);
+template <typename T>
+int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra);
+template <typename T>
+int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, const T *d_in, T *d_out,
                  const double *d_means, int ncols, int64_t col_stride, const int *d_active);
 // dynamic shared memory of a cluster four-step CTA, and the largest a B200 CTA may use
 template <typename T>

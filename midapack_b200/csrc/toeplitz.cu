@@ -1119,7 +1119,7 @@ template <> struct SplitShape<double> { static constexpr int CW = 16, RP = 2, M1
 struct TileCand {
     int log_ml, C, threads;
     int split = 0, log_m1 = 0, log_m2 = 0;  // split plan: M = 2^log_m1 * 2^log_m2
-                                            // (split 2: cluster four-step, M = 2C x 4096)
+                                            // (split 2: cluster four-step, M = 2C x 4096; 3: right-angle)
 };
 
 static int64_t cand_N(const TileCand &c) {
@@ -1128,7 +1128,9 @@ static int64_t cand_N(const TileCand &c) {
 }
 // the split plans (1 and 2) keep one output fewer than the band allows, so that
 // every window starts on an even row
-static int64_t cand_E(const TileCand &c, int lambda) { return cand_N(c) - 2LL * (lambda - 1) - (c.split ? 1 : 0); }
+static int64_t cand_E(const TileCand &c, int lambda) {
+    return cand_N(c) - 2LL * (lambda - 1) - (c.split == 1 || c.split == 2 ? 1 : 0);
+}
 
 // split plans: columns of 16 <= M1 <= 2^m1max points, rows of 32 <= M2 <= 512
 // points; shapes whose transforms end in a lone radix-2 pass (5 or 9 bits) are
@@ -1152,34 +1154,41 @@ static int ceil_log2_i(int64_t v) {
     return b;
 }
 
-// The cluster four-step tiles are candidates of the automatic choice (the
-// autotuner times them with the others).
-static const bool g_cluster4_auto = true;
-
-// every launchable configuration whose tile holds the band (E >= 1)
+// The configurations whose tile holds the band (E >= 1) that the automatic choice
+// considers: every right-angle shape, and the one-CTA tiles of up to 2^8 points
+// for blocks and bands shorter than the smallest right-angle tile.  The longer
+// one-kernel tiles, the split and the cluster four-step tiles were slower than the
+// best right-angle tile at every size timed (blocks of 500 to 2^23 samples, half
+// bandwidths 20 to 2^14, e.g. 64 x 2^20 samples, 2^14: FP64 1.64 -> 1.45 ms, FP32
+// 0.94 -> 0.71 ms; 8 x 2^23, 8192: 1.48 -> 1.26, 0.82 -> 0.64 ms; at the small end
+// 2000 x 500 samples, 20: 38 -> 25 us); they remain plans by name.
 template <typename T>
 static std::vector<TileCand> tile_candidates(int lambda) {
+    std::vector<TileCand> out;
+    for (int lml = 6; lml <= 8; lml++) {
+        TileCand c{lml, 1, default_threads(lml)};
+        if (cand_E(c, lambda) >= 1) out.push_back(c);
+    }
+    for (int a = 0; a <= 4; a++)
+        for (int b = 9; b <= 12; b++) {
+            TileCand c{0, 0, 0, 3, a, b};
+            if (rtile_shape(a, b) && cand_E(c, lambda) >= 1) out.push_back(c);
+        }
+    return out;
+}
+
+// one-kernel tiles of n real samples (plans "fft:n")
+template <typename T>
+static std::vector<TileCand> one_kernel_candidates(int lambda, int64_t n) {
     constexpr int         LMAX = TileLimits<T>::LMAX;
     std::vector<TileCand> out;
     for (int lml = 6; lml <= LMAX; lml++)
         for (int C = 1; C <= 8; C <<= 1) {
             if (C > 1 && lml < LMAX - 1) continue;
-            const int64_t N = 2LL * C * (1LL << lml);
-            if (N - 2LL * (lambda - 1) < 1) continue;
-            out.push_back({lml, C, default_threads(lml)});
-            if (default_threads(lml) == 512) out.push_back({lml, C, 256});  // 2 CTAs per SM when registers allow
-        }
-    for (int logM = 9; logM <= 17; logM++)
-        for (auto ab : split_shapes(logM, SplitShape<T>::M1MAX)) {
-            TileCand c{0, 0, 0, 1, ab.first, ab.second};
-            if (cand_E(c, lambda) < 1) continue;
+            TileCand c{lml, C, default_threads(lml)};
+            if (cand_N(c) != n || cand_E(c, lambda) < 1) continue;
             out.push_back(c);
-        }
-    if (g_cluster4_auto)
-        for (int C = 2; C <= 8; C <<= 1) {  // cluster four-step tiles of 2C x 4096 points
-            TileCand c{13, C, 256, 2, 0, 12};
-            if (cand_E(c, lambda) < 1 || ninv4_smem<T>(C) > NINV4_SMEM_MAX) continue;
-            out.push_back(c);
+            if (c.threads == 512) out.push_back({lml, C, 256});  // 2 CTAs per SM when registers allow
         }
     return out;
 }
@@ -1192,10 +1201,8 @@ static double tile_model_cost(const TileCand &c, int lambda, int64_t max_block) 
     const int     logN = ceil_log2_i(N);
     const double  eff = (double) std::min<int64_t>(E, std::max<int64_t>(max_block, 1));
     double        cost = (double) N / eff * (logN + 3);
-    if (c.split == 2) {
-        cost *= 0.6;  // the tile stays on chip; paired-lane arithmetic
-    } else if (c.split) {
-        cost *= 1.3;  // scratch round trips; the timed choice decides
+    if (c.split == 3) {
+        cost *= c.log_m1 ? 0.5 : 0.4;  // no untangle, paired-lane arithmetic; scratch round trips of the columns
     } else {
         if (c.C > 1) cost += 3.0 * std::log2((double) c.C);
         if (c.threads != default_threads(c.log_ml)) cost *= 1.01;  // ties go to the default launch shape
@@ -1211,14 +1218,16 @@ static int launch_tiles(mdp_context *ctx, const mdp_noise *N, const mdp_tile_pla
                         const double *d_means, int ncols = 1, int64_t col_stride = 0, const int *d_active = nullptr);
 
 // Autotuner.  The plans of a precision are keyed by the band (ceil log2 of
-// lambda) and the block length (ceil log2); the first noise operator with a
+// lambda), the block length (ceil log2) and the rows (ceil log2, at most 2^24: a few
+// tiles leave most of the device idle, where shorter tiles win); the first noise operator with a
 // new key times every candidate kept by the screen below on a sample of its
 // own blocks (at most 2^24 rows, zero data: the tile kernels do the same work
 // whatever the values) and the fastest per useful row is kept for the process.
 struct TuneKey {
-    int prec, lam_bits, blk_bits, device;
+    int prec, lam_bits, blk_bits, row_bits, device;
     bool operator<(const TuneKey &o) const {
-        return std::tie(prec, lam_bits, blk_bits, device) < std::tie(o.prec, o.lam_bits, o.blk_bits, o.device);
+        return std::tie(prec, lam_bits, blk_bits, row_bits, device) <
+               std::tie(o.prec, o.lam_bits, o.blk_bits, o.row_bits, o.device);
     }
 };
 static std::mutex                   g_tune_mu;
@@ -1300,8 +1309,8 @@ static int tune_plan(mdp_context *ctx, const mdp_noise *N, const std::vector<Til
 }
 
 // A plan given by name (mdp_noise_set_plan): "log2_ml,cluster,threads"
-// (one-kernel tiles), "s,log_m1,log_m2" (split tiles) or "c,cluster" (cluster
-// four-step tiles).
+// (one-kernel tiles), "s,log_m1,log_m2" (split tiles), "c,cluster" (cluster
+// four-step tiles) or "r,log_m1,log_m2" (right-angle tiles).
 template <typename T>
 static int parse_plan(const char *plan, int lambda, TileCand *out) {
     TileCand c{0, 0, 0};
@@ -1310,6 +1319,9 @@ static int parse_plan(const char *plan, int lambda, TileCand *out) {
         c.split = 1;
         ok = sscanf(plan + 1, ",%d,%d", &c.log_m1, &c.log_m2) == 2 && c.log_m1 >= 4 &&
              c.log_m1 <= SplitShape<T>::M1MAX && c.log_m2 >= 5 && c.log_m2 <= 9;
+    } else if (plan[0] == 'r') {
+        c.split = 3;
+        ok = sscanf(plan + 1, ",%d,%d", &c.log_m1, &c.log_m2) == 2 && rtile_shape(c.log_m1, c.log_m2);
     } else if (plan[0] == 'c') {
         c = TileCand{13, 0, 256, 2, 0, 12};
         ok = sscanf(plan + 1, ",%d", &c.C) == 1 && (c.C == 2 || c.C == 4 || c.C == 8) &&
@@ -1335,13 +1347,7 @@ static int choose_plan(mdp_context *ctx, const mdp_noise *N, TileCand *out, int 
                        int64_t forced = 0) {
     const bool f32 = sizeof(T) == 4;
     *tuned = 0;
-    std::vector<TileCand> cands = tile_candidates<T>(N->lambda);
-    if (forced) {
-        std::vector<TileCand> keep;
-        for (const TileCand &c : cands)
-            if (cand_N(c) == forced && !c.split) keep.push_back(c);
-        cands.swap(keep);
-    }
+    std::vector<TileCand> cands = forced ? one_kernel_candidates<T>(N->lambda, forced) : tile_candidates<T>(N->lambda);
     if (cands.empty()) return MDP_EUNSUPPORTED;
     std::sort(cands.begin(), cands.end(), [&](const TileCand &a, const TileCand &b) {
         return tile_model_cost(a, N->lambda, N->max_block) < tile_model_cost(b, N->lambda, N->max_block);
@@ -1356,7 +1362,7 @@ static int choose_plan(mdp_context *ctx, const mdp_noise *N, TileCand *out, int 
     }
     if (screen.size() <= 1) return MDP_OK;
     const TuneKey key{f32 ? 32 : 64, ceil_log2(N->lambda), ceil_log2(std::max<int64_t>(N->max_block, 1)),
-                      ctx->device};
+                      std::min(24, ceil_log2(std::max<int64_t>(N->nrow_end, 1))), ctx->device};
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto                        it = g_tuned.find(key);
     if (it != g_tuned.end()) {
@@ -1598,6 +1604,15 @@ static int build_plan(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, const Ti
         P.ready = 1;
         return MDP_OK;
     }
+    if (c.split == 3) {
+        // one row: a one-CTA tile of 2^log_m2 points; several: reported as a split plan
+        P.cluster = c.log_m1 ? 0 : 1;
+        P.log2_ml = c.log_m1 ? 0 : c.log_m2;
+        P.threads = 1 << (c.log_m2 - 4);
+        MDP_TRY(rtile_build<T>(ctx, N, P, spectra));
+        P.ready = 1;
+        return MDP_OK;
+    }
     if (c.split) {
         P.cluster = 0;
         P.threads = 0;
@@ -1649,6 +1664,7 @@ static int launch_tiles(mdp_context *ctx, const mdp_noise *N, const mdp_tile_pla
     if (P.n_tiles == 0 || ncols < 1) return MDP_OK;
     if (ncols > 65535) return MDP_EUNSUPPORTED;
     if (P.split == 2) return ninv4_launch<T>(ctx, N, P, d_in, d_out, d_means, ncols, col_stride, d_active);
+    if (P.split == 3) return rtile_launch<T>(ctx, N, P, d_in, d_out, d_means, ncols, col_stride, d_active);
     if (P.split) return launch_split<T>(ctx, N, P, d_in, d_out, d_means, ncols, col_stride, d_active);
     TileArgsT<T> a;
     a.vin = d_in;
@@ -2146,7 +2162,7 @@ extern "C" int mdp_noise_plan(mdp_context *ctx, mdp_noise *N, int fp32, int *log
     if (threads) *threads = P.threads;
     if (tuned) *tuned = P.tuned;
     if (split_log_m1) *split_log_m1 = P.split ? (P.split == 2 ? 1 + (P.cluster == 8 ? 3 : P.cluster == 4 ? 2 : 1) : P.log_m1) : 0;
-    if (split_log_m2) *split_log_m2 = P.split ? P.log_m2 : 0;
+    if (split_log_m2) *split_log_m2 = P.split ? P.log_m2 : 0;  // (right-angle tiles of one row: log_m1 = 0)
     return MDP_OK;
 }
 
