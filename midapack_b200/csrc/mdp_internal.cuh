@@ -293,6 +293,25 @@ int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_n
 int mdp_trmatvec32_launch(mdp_context *ctx, mdp_pointing *A, const float *d_y, double *d_x);
 int mdp_matvec32_launch(mdp_context *ctx, mdp_pointing *A, const double *d_x, float *d_y);
 
+// Sums of the last block of a two-level reduction: out[k] = the sum of part(k)[0..nb), k < K,
+// in a fixed order (lane l of warp k mod W takes l, l + 32, ..., then the lanes pairwise), valid
+// after the call on every thread (sh: K doubles of shared memory).  One thread adding the
+// partials one after the other waits for an L2 load per addition: 296 partials took 10 us a
+// sum, most of the time of the PCG vector kernels on maps of up to 10^5 pixels (49152
+// pixels: update 33.7 us, dot 13.7 us).
+template <typename F>
+__device__ __forceinline__ void sum_parts(F part, int nb, int K, double *sh) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int k = threadIdx.x >> 5; k < K; k += nw) {
+        const double *p = part(k);
+        double        s = 0.0;
+        for (int b = lane; b < nb; b += 32) s += __ldcg(p + b);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sh[k] = s;
+    }
+    __syncthreads();
+}
+
 inline int grid_for(int64_t n, int threads, int max_blocks = 148 * 16) {
     int64_t b = (n + threads - 1) / threads;
     if (b > max_blocks) b = max_blocks;

@@ -56,7 +56,7 @@ struct MRed {
 
 // ---------------------------------------------------------------- reductions
 // Each block stores K*G partial sums; the last block to finish adds them in
-// block order (deterministic).
+// a fixed order (sum_parts).
 template <int KG>
 __device__ __forceinline__ void mr_block_store(double (&v)[KG], MRed *R) {
     __shared__ double sh[KG][MR_THREADS / 32];
@@ -83,10 +83,12 @@ __device__ __forceinline__ bool mr_last_block(MRed *R, int c) {
     return is_last;
 }
 
-__device__ __forceinline__ double mr_sum(const MRed *R, int k) {
-    double s = 0.0;
-    for (int b = 0; b < MR_BLOCKS; b++) s += R->part[k][b];
-    return s;
+// t[k] = the grid's sum k, k < K (the last block, all its threads)
+template <int K>
+__device__ __forceinline__ const double *mr_sums(const MRed *R) {
+    __shared__ double t[K];
+    sum_parts([R](int k) { return R->part[k]; }, MR_BLOCKS, K, t);
+    return t;
 }
 
 // ---------------------------------------------------------------- operator kernels
@@ -286,10 +288,12 @@ __global__ void __launch_bounds__(MR_THREADS) mr_coeff_kernel(const double *__re
         for (int j = 0; j < G; j++) v[j] += h[3 * j] * q[3 * j] + h[3 * j + 1] * q[3 * j + 1] + h[3 * j + 2] * q[3 * j + 2];
     }
     mr_block_store<G>(v, R);
-    if (mr_last_block(R, 0) && threadIdx.x == 0) {
+    if (mr_last_block(R, 0)) {
+        const double *t = mr_sums<G>(R);
+        if (threadIdx.x != 0) return;
         for (int j = 0; j < G; j++)
             if (run[j]) {
-                S[j].coeff = mr_sum(R, j);
+                S[j].coeff = t[j];
                 S[j].ro = S[j].g2pix / S[j].coeff;
             }
         R->count[0] = 0;
@@ -346,14 +350,16 @@ __global__ void __launch_bounds__(MR_THREADS) mr_update_kernel(const double *__r
         }
     }
     mr_block_store<3 * G>(v, R);
-    if (mr_last_block(R, 1) && threadIdx.x == 0) {
+    if (mr_last_block(R, 1)) {
+        const double *t = mr_sums<3 * G>(R);
+        if (threadIdx.x != 0) return;
         for (int j = 0; j < G; j++) {
             if (!run[j]) continue;
             SlotScal &s = S[j];
             s.g2pixp = s.g2pix;
-            s.g2pix = mr_sum(R, j);
-            s.g2pix_polak = mr_sum(R, G + j);
-            s.res = mr_sum(R, 2 * G + j);
+            s.g2pix = t[j];
+            s.g2pix_polak = t[G + j];
+            s.res = t[2 * G + j];
             s.gamma = s.g2pix_polak / s.g2pixp;
             s.inner_it++;
             s.budget--;
@@ -400,10 +406,12 @@ __global__ void __launch_bounds__(MR_THREADS) mr_slot_init_kernel(const double *
         v[1] += g0 * g0 + g1 * g1 + g2 * g2;
     }
     mr_block_store<2>(v, R);
-    if (mr_last_block(R, 2) && threadIdx.x == 0) {
+    if (mr_last_block(R, 2)) {
+        const double *t = mr_sums<2>(R);
+        if (threadIdx.x != 0) return;
         SlotScal &s = S[j];
-        s.g2pix = mr_sum(R, 0);
-        s.res = mr_sum(R, 1);
+        s.g2pix = t[0];
+        s.res = t[1];
         s.rin0 = s.res;
         s.tol2 = tol2;
         s.cont = 0;  // h = Cg already: no direction update before the first iteration
@@ -439,8 +447,10 @@ __global__ void __launch_bounds__(MR_THREADS) mr_dot_kernel(const double *__rest
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
         v[0] += g[i] * g[i];
     mr_block_store<1>(v, R);
-    if (mr_last_block(R, 3) && threadIdx.x == 0) {
-        S[j].dot = mr_sum(R, 0);
+    if (mr_last_block(R, 3)) {
+        const double *t = mr_sums<1>(R);
+        if (threadIdx.x != 0) return;
+        S[j].dot = t[0];
         R->count[3] = 0;
     }
 }

@@ -8,7 +8,7 @@
 //
 // Device layout: map-domain vectors are contiguous FP64 arrays of n = 3*npix
 // unknowns; the 3x3 blocks are row-major [npix][9].  Dot products are
-// deterministic two-level reductions (fixed grid, partials summed in block
+// deterministic two-level reductions (fixed grid, partials summed in a fixed
 // order by the last block to finish); P^T and the block-Jacobi blocks add
 // their terms in a fixed order too (map bins, below and in pointing.cu), so a
 // solve on pointings of 2^20 rows or more is bitwise reproducible.
@@ -466,7 +466,7 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[K], Scal *S, int 
         }
 }
 
-// last block to finish sums the partials in block order (deterministic)
+// the last block to finish sums the partials (sum_parts: a fixed order)
 __device__ __forceinline__ bool last_block(Scal *S, int slot) {
     __shared__ bool is_last;
     __threadfence();
@@ -480,10 +480,12 @@ __device__ __forceinline__ bool last_block(Scal *S, int slot) {
     return is_last;
 }
 
-__device__ __forceinline__ double sum_partials(const Scal *S, int slot) {
-    double s = 0.0;
-    for (int b = 0; b < (int) gridDim.x; b++) s += ((volatile const Scal *) S)->partial[slot][b];
-    return s;
+// t[k] = the grid's sum k, k < K (the last block, all its threads)
+template <int K>
+__device__ __forceinline__ const double *sum_partials(const Scal *S) {
+    __shared__ double t[K];
+    sum_parts([S](int k) { return S->partial[k]; }, (int) gridDim.x, K, t);
+    return t;
 }
 
 // RHS: _g = b + noise - P x0 with x0 = 0; cut rows have b zeroed (precond.c:605-615)
@@ -521,9 +523,11 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_init_kernel(const double *__r
         v[1] += g0 * g0 + g1 * g1 + g2 * g2;
     }
     block_reduce_store<2>(v, S, 0);
-    if (last_block(S, 0) && threadIdx.x == 0) {
-        S->g2pix = sum_partials(S, 0);
-        S->res = sum_partials(S, 1);
+    if (last_block(S, 0)) {
+        const double *t = sum_partials<2>(S);
+        if (threadIdx.x != 0) return;
+        S->g2pix = t[0];
+        S->res = t[1];
         S->count[0] = 0;
     }
 }
@@ -535,8 +539,10 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_coeff_kernel(const double *__
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
         v[0] += h[i] * q_[i];
     block_reduce_store<1>(v, S, 0);
-    if (last_block(S, 1) && threadIdx.x == 0) {
-        S->coeff = sum_partials(S, 0);
+    if (last_block(S, 1)) {
+        const double *t = sum_partials<1>(S);
+        if (threadIdx.x != 0) return;
+        S->coeff = t[0];
         S->ro = S->g2pix / S->coeff;
         S->count[1] = 0;
     }
@@ -574,11 +580,13 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_update_kernel(const double *_
         }
     }
     block_reduce_store<3>(v, S, 0);
-    if (last_block(S, 2) && threadIdx.x == 0) {
+    if (last_block(S, 2)) {
+        const double *t = sum_partials<3>(S);
+        if (threadIdx.x != 0) return;
         S->g2pixp = S->g2pix;
-        S->g2pix = sum_partials(S, 0);
-        S->g2pix_polak = sum_partials(S, 1);
-        S->res = sum_partials(S, 2);
+        S->g2pix = t[0];
+        S->g2pix_polak = t[1];
+        S->res = t[2];
         S->gamma = S->g2pix_polak / S->g2pixp;
         S->count[2] = 0;
     }
@@ -636,9 +644,11 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_init_tl_kernel(const double *
         }
     }
     block_reduce_store<2>(v, S, 0);
-    if (last_block(S, 0) && threadIdx.x == 0) {
-        S->g2pix = sum_partials(S, 0);
-        S->res = sum_partials(S, 1);
+    if (last_block(S, 0)) {
+        const double *t = sum_partials<2>(S);
+        if (threadIdx.x != 0) return;
+        S->g2pix = t[0];
+        S->res = t[1];
         S->count[0] = 0;
     }
 }
@@ -679,11 +689,13 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_precond_tl_kernel(const doubl
         }
     }
     block_reduce_store<3>(v, S, 0);
-    if (last_block(S, 2) && threadIdx.x == 0) {
+    if (last_block(S, 2)) {
+        const double *t = sum_partials<3>(S);
+        if (threadIdx.x != 0) return;
         S->g2pixp = S->g2pix;
-        S->g2pix = sum_partials(S, 0);
-        S->g2pix_polak = sum_partials(S, 1);
-        S->res = sum_partials(S, 2);
+        S->g2pix = t[0];
+        S->g2pix_polak = t[1];
+        S->res = t[2];
         S->gamma = S->g2pix_polak / S->g2pixp;
         S->count[2] = 0;
     }
@@ -708,8 +720,10 @@ __global__ void __launch_bounds__(RED_THREADS) dot_self_kernel(const double *__r
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
         v[0] += g[i] * g[i];
     block_reduce_store<1>(v, S, 0);
-    if (last_block(S, 3) && threadIdx.x == 0) {
-        S->res = sum_partials(S, 0);
+    if (last_block(S, 3)) {
+        const double *t = sum_partials<1>(S);
+        if (threadIdx.x != 0) return;
+        S->res = t[0];
         S->count[3] = 0;
     }
 }

@@ -98,16 +98,11 @@ __global__ void sum_partials_kernel(const double *__restrict__ part, int nb, int
     }
 }
 
-// qtx = Em1 (Z^T g): w[j] from the partials in block order, then the small product (precond.c:1036-1051)
+// qtx = Em1 (Z^T g): w[j] from the partials in a fixed order, then the small product (precond.c:1036-1051)
 __global__ void qtx_kernel(const double *__restrict__ part, int nb, const double *__restrict__ Em1, int zn,
                            double *__restrict__ qtx) {
     __shared__ double w[MDP_TL_MAX_ZN];
-    for (int j = threadIdx.x; j < zn; j += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nb; b++) s += part[(int64_t) j * nb + b];
-        w[j] = s;
-    }
-    __syncthreads();
+    sum_parts([part, nb](int j) { return part + (int64_t) j * nb; }, nb, zn, w);
     for (int i = threadIdx.x; i < zn; i += blockDim.x) {
         double s = 0.0;
         for (int j = 0; j < zn; j++) s += Em1[i * zn + j] * w[j];
