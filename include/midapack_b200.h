@@ -132,8 +132,9 @@ int  mdp_noise_set_plan(mdp_context *ctx, mdp_noise *N, int fp32, const char *pl
  * a plugin that may only touch buffers its host gives it).  The block-mean
  * scratch lives in a fixed 1 MiB device array (131072 doubles) that the library
  * keeps on every device it is loaded on until the process exits; a noise
- * operator needing more (one double per block plus one per 65536-row chunk of
- * every block) is rejected with MDP_EINVAL, as is d_in == d_out.  The first
+ * operator needing more (one double per block plus one per row chunk of every
+ * block; 65536 rows a chunk, down to 2048 in operators that would have few
+ * chunks) is rejected with MDP_EINVAL, as is d_in == d_out.  The first
  * call on a device looks up that array's device address (once per device), so
  * make the first call before any stream capture.  The cached address belongs
  * to the device's primary context (the runtime's): calls from another context

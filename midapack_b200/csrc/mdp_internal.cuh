@@ -202,7 +202,7 @@ struct mdp_noise {
     std::vector<double>  h_Tuniq;        // [n_spec][lambda] distinct first rows
     mdp_tile_plan        p64;            // built at creation
     mdp_tile_plan        p32;            // built on first FP32 use
-    // 65536-row chunks of the deterministic block-mean reduction
+    // chunks (2048 to 65536 rows) of the deterministic block-mean reduction
     int                  n_chunks = 0;
     bool                 covers_all = true;  // blocks tile rows [0, nrow_end) without holes
     DevBuf               chunk_start;    // int64 [n_chunks]

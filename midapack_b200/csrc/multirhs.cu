@@ -93,7 +93,7 @@ __device__ __forceinline__ const double *mr_sums(const MRed *R) {
 
 // ---------------------------------------------------------------- operator kernels
 // Y[j] = P h_j (FP32 weights, FP32 copy of h_j) for the running slots, with
-// FP64 partial sums per 65536-row chunk (block means of N^-1).  The FP32 copy
+// FP64 partial sums per row chunk (block means of N^-1).  The FP32 copy
 // of the slot directions (12 bytes per pixel and slot) keeps the gathered map
 // L2-resident for 8 slots of a few million pixels.
 template <int G>
@@ -172,14 +172,18 @@ __global__ void __launch_bounds__(512) mr_matvec32_kernel(const int32_t *__restr
     }
 }
 
+// block means of every slot from its chunk sums, a warp a block
 __global__ void mr_means_kernel(const double *__restrict__ partial, int n_chunks, const int32_t *__restrict__ blk_chunk0,
                                 const int32_t *__restrict__ blk_nchunk, const int32_t *__restrict__ blk_len, int nb,
                                 double *__restrict__ means) {
-    const int j = blockIdx.y;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int c = 0; c < blk_nchunk[b]; c++) s += partial[(int64_t) j * n_chunks + blk_chunk0[b] + c];
-        means[(int64_t) j * nb + b] = s / (double) blk_len[b];
+    const int j = blockIdx.y, lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nw) {
+        const int     n = blk_nchunk[b];
+        const double *p = partial + (int64_t) j * n_chunks + blk_chunk0[b];
+        double        s = 0.0;
+        for (int c = lane; c < n; c += 32) s += p[c];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) means[(int64_t) j * nb + b] = s / (double) blk_len[b];
     }
 }
 
@@ -480,7 +484,7 @@ int launch_apply32(mdp_context *ctx, mdp_pointing *A, mdp_noise *N, Batch &B, co
                                                       B.m, B.chunk_start, B.chunk_len, B.n_chunks,
                                                       B.partial.as<double>());
     MDP_CHECK_LAUNCH(ctx);
-    mr_means_kernel<<<dim3(grid_for(N->nb, 128, 64), G), 128, 0, st>>>(B.partial.as<double>(), B.n_chunks,
+    mr_means_kernel<<<dim3(grid_for(N->nb, 4, 256), G), 128, 0, st>>>(B.partial.as<double>(), B.n_chunks,
                                                                        B.blk_chunk0, B.blk_nchunk,
                                                                        N->blk_len.as<int32_t>(), N->nb,
                                                                        B.means.as<double>());

@@ -1052,14 +1052,24 @@ __global__ void block_partial_sums(const T *__restrict__ v, const int64_t *__res
     }
 }
 
+// the mean of every block from its chunk sums, a warp a block (lane l adds chunks l, l + 32, ...,
+// then the lanes pairwise)
 __global__ void block_means_final(const double *__restrict__ partial, const int32_t *__restrict__ blk_chunk0,
                                   const int32_t *__restrict__ blk_nchunk, const int32_t *__restrict__ blk_len,
                                   int nb, double *__restrict__ means) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int c = 0; c < blk_nchunk[b]; c++) s += partial[blk_chunk0[b] + c];
-        means[b] = s / (double) blk_len[b];
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nw) {
+        const int     n = blk_nchunk[b];
+        const double *p = partial + blk_chunk0[b];
+        double        s = 0.0;
+        for (int c = lane; c < n; c += 32) s += p[c];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) means[b] = s / (double) blk_len[b];
     }
+}
+static void launch_means_final(mdp_context *ctx, const mdp_noise *N, const double *partial, double *means) {
+    block_means_final<<<grid_for(N->nb, 4, 2048), 128, 0, ctx->stream>>>(
+            partial, N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(), N->nb, means);
 }
 
 __global__ void white_kernel(const double *__restrict__ vin, double *__restrict__ vout, const int64_t *__restrict__ bstart,
@@ -1755,8 +1765,13 @@ extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *
     cudaMemcpy(N->blk_len.p, h_n, 4 * nb_blocks, cudaMemcpyHostToDevice);
     cudaMemcpy(N->blk_t0.p, N->h_T0.data(), 8 * nb_blocks, cudaMemcpyHostToDevice);
 
-    // chunks for the deterministic block-mean reduction
-    const int            CH = 1 << 16;
+    // chunks of the deterministic block-mean reduction and of P fused with it, one CTA each:
+    // 65536 rows, halved down to 2048 while there are fewer than eight per SM
+    int CH = 1 << 16;
+    for (int64_t n_ch = 0; CH > 2048; CH >>= 1, n_ch = 0) {
+        for (int b = 0; b < nb_blocks && n_ch < 8 * ctx->sm_count; b++) n_ch += (h_n[b] + (int64_t) CH - 1) / CH;
+        if (n_ch >= 8 * ctx->sm_count) break;
+    }
     std::vector<int64_t> cs;
     std::vector<int32_t> cl, c0(nb_blocks), cn(nb_blocks);
     for (int b = 0; b < nb_blocks; b++) {
@@ -1835,9 +1850,7 @@ int mdp_block_means(mdp_context *ctx, const mdp_noise *N, const double *d_v, dou
     block_partial_sums<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_v, N->chunk_start.as<int64_t>(),
                                                              N->chunk_len.as<int32_t>(), N->partial.as<double>());
     MDP_CHECK_LAUNCH(ctx);
-    block_means_final<<<grid_for(N->nb, 128, 1024), 128, 0, ctx->stream>>>(
-            N->partial.as<double>(), N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(),
-            N->nb, d_means);
+    launch_means_final(ctx, N, N->partial.as<double>(), d_means);
     MDP_CHECK_LAUNCH(ctx);
     return MDP_OK;
 }
@@ -1860,8 +1873,15 @@ int mdp_stbmm_impl(mdp_context *ctx, const mdp_noise *N, const double *d_in, dou
     return launch_tiles<double>(ctx, N, N->p64, d_in, d_out, d_means);
 }
 
-// y = P x fused with the block-mean partial sums of y: one CTA per 65536-row
-// chunk of a block, so the mean-removal pass of N^-1 needs no second read of y.
+// y = P x fused with the block-mean partial sums of y, one CTA per chunk, so the mean-removal
+// pass of N^-1 needs no second read of y.  Two consecutive rows (from an even row on) a
+// thread, their six weights as three 16-byte loads (VEC: weights and output 16-byte aligned;
+// the chunk's odd first and last row by themselves).  Bound: DRAM.  With one row a thread and
+// fixed chunks of 65536 rows, 4 x 2^20 rows ran on 64 CTAs and took 138 us.
+__device__ __forceinline__ double p64_row(int32_t o, double w0, double w1, double w2, const double *__restrict__ x) {
+    return o >= 0 ? w0 * __ldg(x + o) + w1 * __ldg(x + o + 1) + w2 * __ldg(x + o + 2) : 0.0;
+}
+template <bool VEC>
 __global__ void __launch_bounds__(512) matvec_chunk_sums_kernel(const int32_t *__restrict__ off,
                                                                 const double *__restrict__ w,
                                                                 const double *__restrict__ x, double *__restrict__ y,
@@ -1869,15 +1889,31 @@ __global__ void __launch_bounds__(512) matvec_chunk_sums_kernel(const int32_t *_
                                                                 const int32_t *__restrict__ chunk_len,
                                                                 double *__restrict__ partial) {
     const int64_t s = chunk_start[blockIdx.x];
-    const int     n = chunk_len[blockIdx.x];
+    const int64_t e = s + chunk_len[blockIdx.x];
     double        acc = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const int64_t t = s + j;
-        const int32_t o = off[t];
-        double        v = 0.0;
-        if (o >= 0) v = w[3 * t] * __ldg(x + o) + w[3 * t + 1] * __ldg(x + o + 1) + w[3 * t + 2] * __ldg(x + o + 2);
-        y[t] = v;
-        acc += v;
+    if constexpr (VEC) {
+        const int64_t a = min((s + 1) & ~(int64_t) 1, e), b = max(e & ~(int64_t) 1, a);
+        for (int64_t t = a + 2 * (int64_t) threadIdx.x; t < b; t += 2 * (int64_t) blockDim.x) {
+            const int2     o = __ldg(reinterpret_cast<const int2 *>(off + t));
+            const double2 *wv = reinterpret_cast<const double2 *>(w + 3 * t);
+            const double2  w0 = __ldg(wv), w1 = __ldg(wv + 1), w2 = __ldg(wv + 2);
+            const double2  v = make_double2(p64_row(o.x, w0.x, w0.y, w1.x, x), p64_row(o.y, w1.y, w2.x, w2.y, x));
+            *reinterpret_cast<double2 *>(y + t) = v;
+            acc += v.x + v.y;
+        }
+        const int64_t rest = (a - s) + (e - b);  // 0, 1 or 2 rows
+        if (threadIdx.x < rest) {
+            const int64_t t = threadIdx.x < a - s ? s : b;
+            const double  v = p64_row(off[t], w[3 * t], w[3 * t + 1], w[3 * t + 2], x);
+            y[t] = v;
+            acc += v;
+        }
+    } else {
+        for (int64_t t = s + threadIdx.x; t < e; t += blockDim.x) {
+            const double v = p64_row(off[t], w[3 * t], w[3 * t + 1], w[3 * t + 2], x);
+            y[t] = v;
+            acc += v;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     __shared__ double ws[16];
@@ -1897,13 +1933,12 @@ int mdp_matvec_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noi
                           double *d_y) {
     if (!A->triplet || !N->covers_all || N->lambda == 1 || N->nrow_end != A->m || N->n_chunks == 0)
         return MDP_EUNSUPPORTED;
-    matvec_chunk_sums_kernel<<<N->n_chunks, 512, 0, ctx->stream>>>(A->off.as<int32_t>(), A->values, d_x, d_y,
-                                                                   N->chunk_start.as<int64_t>(),
-                                                                   N->chunk_len.as<int32_t>(), N->partial.as<double>());
+    const bool vec = ((reinterpret_cast<uintptr_t>(A->values) | reinterpret_cast<uintptr_t>(d_y)) & 15) == 0;
+    (vec ? matvec_chunk_sums_kernel<true> : matvec_chunk_sums_kernel<false>)<<<N->n_chunks, 512, 0, ctx->stream>>>(
+            A->off.as<int32_t>(), A->values, d_x, d_y, N->chunk_start.as<int64_t>(), N->chunk_len.as<int32_t>(),
+            N->partial.as<double>());
     MDP_CHECK_LAUNCH(ctx);
-    block_means_final<<<grid_for(N->nb, 128, 1024), 128, 0, ctx->stream>>>(
-            N->partial.as<double>(), N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(),
-            N->nb, N->means.as<double>());
+    launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
     MDP_CHECK_LAUNCH(ctx);
     return MDP_OK;
 }
@@ -1948,9 +1983,7 @@ int mdp_stbmm_impl32(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d
             block_partial_sums<float><<<N->n_chunks, 512, 0, ctx->stream>>>(
                     d_in, N->chunk_start.as<int64_t>(), N->chunk_len.as<int32_t>(), N->partial.as<double>());
             MDP_CHECK_LAUNCH(ctx);
-            block_means_final<<<grid_for(N->nb, 128, 1024), 128, 0, ctx->stream>>>(
-                    N->partial.as<double>(), N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(),
-                    N->blk_len.as<int32_t>(), N->nb, N->means.as<double>());
+            launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
             MDP_CHECK_LAUNCH(ctx);
         }
         d_means = N->means.as<double>();
@@ -1968,7 +2001,7 @@ int mdp_stbmm32_batch(mdp_context *ctx, mdp_noise *N, const float *d_in, float *
     return launch_tiles<float>(ctx, N, N->p32, d_in, d_out, d_means, ncols, col_stride, d_active);
 }
 
-// chunks of the block-mean reduction (65536 rows each, in block order)
+// chunks of the block-mean reduction (2048 to 65536 rows each, in block order)
 int mdp_noise_chunks(const mdp_noise *N, int *n_chunks, const int64_t **d_chunk_start, const int32_t **d_chunk_len,
                      const int32_t **d_blk_chunk0, const int32_t **d_blk_nchunk, int *covers_all) {
     *n_chunks = N->n_chunks;
@@ -2092,9 +2125,7 @@ int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_n
                 N->chunk_len.as<int32_t>(), N->partial.as<double>());
     }
     MDP_CHECK_LAUNCH(ctx);
-    block_means_final<<<grid_for(N->nb, 128, 1024), 128, 0, ctx->stream>>>(
-            N->partial.as<double>(), N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(),
-            N->nb, N->means.as<double>());
+    launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
     MDP_CHECK_LAUNCH(ctx);
     return MDP_OK;
 }
@@ -2237,7 +2268,7 @@ extern "C" int mdp_stbmm_noalloc(mdp_context *ctx, const mdp_noise *N, const dou
     }
     const int64_t need = (int64_t) N->n_chunks + N->nb;
     if (N->lambda > 1 && need > MDP_NOALLOC_SCRATCH_DOUBLES) {
-        mdp_set_error("mdp_stbmm_noalloc: %lld scratch doubles needed (%d blocks, %d 65536-row chunks), limit %d",
+        mdp_set_error("mdp_stbmm_noalloc: %lld scratch doubles needed (%d blocks, %d row chunks), limit %d",
                       (long long) need, N->nb, N->n_chunks, MDP_NOALLOC_SCRATCH_DOUBLES);
         return MDP_EINVAL;
     }
@@ -2251,9 +2282,7 @@ extern "C" int mdp_stbmm_noalloc(mdp_context *ctx, const mdp_noise *N, const dou
         block_partial_sums<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunk_start.as<int64_t>(),
                                                                  N->chunk_len.as<int32_t>(), partial);
         MDP_CHECK_LAUNCH(ctx);
-        block_means_final<<<grid_for(N->nb, 128, 1024), 128, 0, ctx->stream>>>(
-                partial, N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(), N->nb,
-                means);
+        launch_means_final(ctx, N, partial, means);
         MDP_CHECK_LAUNCH(ctx);
     } else {
         MDP_CUDA(cudaMemsetAsync(means, 0, sizeof(double) * N->nb, ctx->stream));
