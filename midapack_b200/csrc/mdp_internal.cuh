@@ -280,6 +280,10 @@ size_t ninv4_smem(int C);
 #define NINV4_SMEM_MAX ((size_t) 227 * 1024)
 int mdp_matvec_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noise *N, const double *d_x,
                           double *d_y);
+// periodograms of long blocks (psd.cu): whether it takes a length, and the blocks idx of a call
+bool mdp_psd_takes(int64_t n);
+int mdp_psd_blocks(mdp_context *ctx, const std::vector<int> &idx, const int32_t *n, const std::vector<int64_t> &at,
+                   const std::vector<int64_t> &out, const double *d_x, double fsamp, double *d_psd);
 // FP32 operator pieces (mixed precision)
 int mdp_noise_prepare_fp32(mdp_context *ctx, mdp_noise *N);
 int mdp_stbmm_impl32(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d_out, const double *d_means);

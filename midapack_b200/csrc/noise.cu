@@ -703,12 +703,26 @@ extern "C" int mdp_periodogram(mdp_context *ctx, int nb, const int32_t *h_n, con
     std::vector<Batch> batches;
     std::vector<int64_t> offs;
     MDP_TRY(make_batches(nb, h_n, 4, &batches, &offs));
+    // blocks whose transform is longer than one CTA's: all of a length together (psd.cu)
+    std::vector<int64_t> outs(nb);
+    std::vector<int>     longer;
+    int64_t              at = 0;
+    for (int b = 0; b < nb; ++b) {
+        outs[b] = at;
+        at += h_n[b] / 2 + 1;
+        if (mdp_psd_takes(h_n[b])) longer.push_back(b);
+    }
+    if (!longer.empty()) MDP_TRY(mdp_psd_blocks(ctx, longer, h_n, offs, outs, d_noise, fsamp, d_psd));
+    if ((int) longer.size() == nb) {
+        MDP_CUDA(cudaStreamSynchronize(ctx->stream));
+        return MDP_OK;
+    }
     MDP_TRY(set_fft_smem());
     DevBuf buf, bh, part, sums, doff, flag;
     MDP_TRY(flag.alloc(sizeof(int)));
-    int64_t psd_at = 0;
     int64_t bh_n = -1;
     for (const Batch &bt : batches) {
+        if (mdp_psd_takes(bt.n)) continue;
         FftShape sh;
         int blue;
         MDP_TRY(shape_for(bt.n, &sh, &blue));
@@ -722,9 +736,8 @@ extern "C" int mdp_periodogram(mdp_context *ctx, int nb, const int32_t *h_n, con
             bh_n = bt.n;
         }
         MDP_TRY(periodogram_batch(ctx, d_noise, doff.as<int64_t>(), bt.cnt, bt.n, sh, blue, bh.as<double2>(),
-                                  buf.as<double2>(), part, sums, fsamp, nullptr, d_psd + psd_at, bt.n / 2 + 1,
+                                  buf.as<double2>(), part, sums, fsamp, nullptr, d_psd + outs[bt.first], bt.n / 2 + 1,
                                   flag.as<int>()));
-        psd_at += (int64_t) bt.cnt * (bt.n / 2 + 1);
         // buffers are reused by the next batch: finish this one first
         MDP_CUDA(cudaStreamSynchronize(ctx->stream));
     }
