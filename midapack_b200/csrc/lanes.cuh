@@ -4,7 +4,7 @@
 // Pr<T> is one real value on every lane of a register set: Pr<float> is two
 // FP32 lanes in one 64-bit register pair (Blackwell's paired add/sub/mul/fma
 // .f32x2, one instruction for both lanes, each rounded as the scalar one),
-// Pr<double> two FP64 lanes, Pr<mono64> a single FP64 lane.  CP<T> is a complex
+// Pr<double> two FP64 lanes, Pr<mono32> and Pr<mono64> a single lane.  CP<T> is a complex
 // value per lane, real and imaginary parts in separate Pr.
 #pragma once
 
@@ -23,6 +23,10 @@ template <> struct Pr<double> {
 struct mono64 {};
 template <> struct Pr<mono64> {
     double v;
+};
+struct mono32 {};
+template <> struct Pr<mono32> {
+    float v;
 };
 
 __device__ __forceinline__ Pr<float> pmk(float a, float b) {
@@ -78,6 +82,11 @@ __device__ __forceinline__ Pr<mono64> psub(Pr<mono64> x, Pr<mono64> y) { return 
 __device__ __forceinline__ Pr<mono64> pmul(Pr<mono64> x, Pr<mono64> y) { return {x.v * y.v}; }
 __device__ __forceinline__ Pr<mono64> pfma(Pr<mono64> x, Pr<mono64> y, Pr<mono64> z) { return {fma(x.v, y.v, z.v)}; }
 
+__device__ __forceinline__ Pr<mono32> padd(Pr<mono32> x, Pr<mono32> y) { return {x.v + y.v}; }
+__device__ __forceinline__ Pr<mono32> psub(Pr<mono32> x, Pr<mono32> y) { return {x.v - y.v}; }
+__device__ __forceinline__ Pr<mono32> pmul(Pr<mono32> x, Pr<mono32> y) { return {x.v * y.v}; }
+__device__ __forceinline__ Pr<mono32> pfma(Pr<mono32> x, Pr<mono32> y, Pr<mono32> z) { return {fmaf(x.v, y.v, z.v)}; }
+
 template <typename T> __device__ __forceinline__ Pr<T> pdup(T s) { return pmk(s, s); }
 // a compile-time constant on both lanes: plain integer bits for FP32 (the
 // compiler may rematerialise it at each use instead of keeping it live)
@@ -88,6 +97,7 @@ template <> __device__ __forceinline__ Pr<float> pcst<float>(double v) {
 }
 template <> __device__ __forceinline__ Pr<double> pcst<double>(double v) { return Pr<double>{v, v}; }
 template <> __device__ __forceinline__ Pr<mono64> pcst<mono64>(double v) { return Pr<mono64>{v}; }
+template <> __device__ __forceinline__ Pr<mono32> pcst<mono32>(double v) { return Pr<mono32>{(float) v}; }
 
 // complex values on both lanes: x = real parts (lane A, lane B), y = imaginary parts
 template <typename T> struct CP {
@@ -96,6 +106,15 @@ template <typename T> struct CP {
 
 template <typename T> __device__ __forceinline__ CP<T> cpadd(CP<T> a, CP<T> b) { return {padd(a.x, b.x), padd(a.y, b.y)}; }
 template <typename T> __device__ __forceinline__ CP<T> cpsub(CP<T> a, CP<T> b) { return {psub(a.x, b.x), psub(a.y, b.y)}; }
+// one FP32 lane: the two components in one paired instruction
+template <> __device__ __forceinline__ CP<mono32> cpadd<mono32>(CP<mono32> a, CP<mono32> b) {
+    const Pr<float> r = padd(pmk(a.x.v, a.y.v), pmk(b.x.v, b.y.v));
+    return {Pr<mono32>{plo(r)}, Pr<mono32>{phi(r)}};
+}
+template <> __device__ __forceinline__ CP<mono32> cpsub<mono32>(CP<mono32> a, CP<mono32> b) {
+    const Pr<float> r = psub(pmk(a.x.v, a.y.v), pmk(b.x.v, b.y.v));
+    return {Pr<mono32>{plo(r)}, Pr<mono32>{phi(r)}};
+}
 // a * w
 template <typename T> __device__ __forceinline__ CP<T> cpmul(CP<T> a, CP<T> w) {
     return {psub(pmul(a.x, w.x), pmul(a.y, w.y)), pfma(a.x, w.y, pmul(a.y, w.x))};

@@ -87,6 +87,10 @@ struct mdp_context {
     // synchronise the device, in the solves of a serving loop
     DevBuf       ws[13];    // [12]: FP32 (x, y, z, 0) copy of the map gathered by the FP32 P
     double      *h_pinned = nullptr;  // pinned host scalars
+    // a second stream for launches that may overlap those on `stream`: forked from it and
+    // joined to it again within one call (mdp_side_fork / mdp_side_join), created on first use
+    cudaStream_t side = nullptr;
+    cudaEvent_t  side_ev[2] = {nullptr, nullptr};
     // optional per-operator timing inside the solver (CUDA events on the stream)
     int          profile = 0;
     double       prof_ms[4] = {0, 0, 0, 0};   // P, N^-1, P^T, vector/dot kernels
@@ -163,7 +167,7 @@ struct mdp_tile_plan {
                            // 2: cluster four-step (ninv4.cu: C = cluster CTAs, M = 2C x 4096 points);
                            // 3: right-angle tiles (rtile.cu, M = 2^log_m1 x 2^log_m2 points)
     int     log_m1 = 0, log_m2 = 0;  // split: M = 2^log_m1 * 2^log_m2 complex points per tile
-    DevBuf  scratch;       // split: [n_tiles][M] complex work array; right-angle tiles: one launch group's
+    DevBuf  scratch;       // split: [n_tiles][M] complex work array; right-angle tiles: two launch groups'
     DevBuf  ltw2, wa, wb;  // split: row-pass twiddles, W_M factor tables
     int     log2_ml = 0;   // per-CTA complex points = 2^log2_ml
     int     cluster = 1;   // CTAs per tile
@@ -171,7 +175,7 @@ struct mdp_tile_plan {
     int     fft_n = 0;     // real FFT size N = 2 * cluster * 2^log2_ml
     int     tuned = 0;     // 1 when picked by timing the candidates on the device
     int64_t n_tiles = 0;
-    DevBuf  tile_start;    // int64 [n_tiles] first output row (global)
+    DevBuf  tile_start;    // int64 [n_tiles] first output row (global); right-angle tiles: mdp_rtile [n_tiles]
     DevBuf  tile_block;    // int32 [n_tiles]
     DevBuf  spectra;       // V [n_spec][N/4+1]: spectrum pairs in tile position order
     DevBuf  ltw, twm, ttw; // packed local-pass, cross-CTA and twist twiddles
@@ -184,6 +188,13 @@ struct mdp_tile_plan {
     }
 };
 
+// window of a right-angle tile (rtile.cu)
+struct alignas(16) mdp_rtile {
+    int64_t start;             // first row of the tile's block
+    int32_t o, len, e;         // window start relative to it, block length, outputs of the tile
+    int32_t spec, blk, unused; // spectrum, block
+};
+
 struct mdp_noise {
     uint64_t             uid = 0;        // unique per created operator
     int                  nb = 0;
@@ -193,6 +204,7 @@ struct mdp_noise {
     std::vector<int64_t> h_idv;
     std::vector<int32_t> h_n;
     std::vector<double>  h_T0;           // diagonal of each block
+    std::vector<int32_t> h_spec;         // spectrum of each block (empty: all the first)
     DevBuf               blk_start;      // int64 [nb]
     DevBuf               blk_len;        // int32 [nb]
     DevBuf               blk_spec;       // int32 [nb] index of the block's spectrum
@@ -249,6 +261,9 @@ int mdp_matvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d_x
 int mdp_trmatvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d_y, double *d_x);
 
 // ---------------------------------------------------------------- helpers (pointing.cu / reduce)
+// ctx->side continues from what ctx->stream holds; ctx->stream waits for ctx->side
+int mdp_side_fork(mdp_context *ctx);
+int mdp_side_join(mdp_context *ctx);
 int mdp_exclusive_scan_u32(mdp_context *ctx, const uint32_t *d_in, uint32_t *d_out, int64_t n,
                            uint32_t *h_total);
 int mdp_stbmm_impl(mdp_context *ctx, const mdp_noise *N, const double *d_in, double *d_out,

@@ -83,6 +83,9 @@ extern "C" void mdp_context_destroy(mdp_context *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    for (cudaEvent_t e : ctx->side_ev)
+        if (e) cudaEventDestroy(e);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     for (int i = 0; i < 5; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
@@ -100,6 +103,22 @@ extern "C" int mdp_context_set_stream(mdp_context *ctx, void *cuda_stream) {
         MDP_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         ctx->own_stream = true;
     }
+    return MDP_OK;
+}
+
+int mdp_side_fork(mdp_context *ctx) {
+    if (!ctx->side) {
+        for (cudaEvent_t &e : ctx->side_ev) MDP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        MDP_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    }
+    MDP_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
+    MDP_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
+    return MDP_OK;
+}
+
+int mdp_side_join(mdp_context *ctx) {
+    MDP_CUDA(cudaEventRecord(ctx->side_ev[1], ctx->side));
+    MDP_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
     return MDP_OK;
 }
 

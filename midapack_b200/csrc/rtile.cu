@@ -28,16 +28,19 @@
 // values with real and imaginary parts exchanged, conj(DFT(conj v)) =
 // swap(DFT(swap v)), a renaming of registers.
 //
-// FP32: two tiles run as the two lanes of the paired FP32 instructions (same
-// twiddles, their own spectra); a shared-memory or scratch entry is 16 bytes, (x_0,
-// x_1, y_0, y_1).  FP64: one tile, an entry is (x, y), 16 bytes too.
+// One tile a CTA (FP32: 16 points take 32 of 64 registers, four CTAs of 256 threads an SM;
+// FP64: 64 of 128, two).  FP32 complex sums are one paired FP32 instruction (add/sub
+// .f32x2) on (x, y).  Two FP32 tiles on the lanes of paired instructions took fewer
+// instructions and half the resident warps: 0.71 against 0.70 ms below, 131 against 94 us for
+// 8 x 2^20 samples at half bandwidth 2^13.
 //
 // Measured against the best of the even/odd-packed plans on a B200 (64 x 2^20 samples,
-// half bandwidth 2^14): FP32 0.93 -> 0.71 ms (60 instead of ~250 thread instructions a
-// complex point in the row kernel), error against 64 bits 5.9e-7 -> 2.6e-7; FP64 1.62 ->
-// 1.46 ms, 1.1e-15 -> 8.7e-16.  A spectrum from the transform itself takes microseconds
-// where the direct cosine sums took 3.7 ms (half bandwidth 2^13, 2^17 samples).
+// half bandwidth 2^14): FP32 0.93 -> 0.645 ms, error against 64 bits 5.9e-7 -> 2.7e-7; FP64
+// 1.62 -> 1.20 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 76 % busy in
+// FP32, waiting for its loads in FP64.  A spectrum from the transform itself takes
+// microseconds where the direct cosine sums took 3.7 ms (half bandwidth 2^13, 2^17 samples).
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "lanes.cuh"
@@ -47,26 +50,24 @@ namespace {
 
 template <typename T> struct LaneOf;
 template <> struct LaneOf<float> {
-    using Tag = float;
+    using Tag = mono32;
     using V2 = float2;
-    static constexpr int N = 2;
 };
 template <> struct LaneOf<double> {
     using Tag = mono64;
     using V2 = double2;
-    static constexpr int N = 1;
 };
 
-template <typename G> struct alignas(16) REnt {  // one complex value per lane
+template <typename G> struct alignas(2 * sizeof(Pr<G>)) REnt {  // a complex value in shared memory or scratch
     Pr<G> x, y;
 };
 
-// where the samples of one lane's tile lie
-template <typename T> struct Lane {
+// where a tile's samples lie
+template <typename T> struct Tile {
     const T *in;   // the block's first sample
     T       *out;
     int      o;    // window start relative to the block
-    int      len;  // block length (0: no tile on this lane)
+    int      len;  // block length
     int      e;    // outputs of the tile inside the block
     T        mu;
 };
@@ -79,92 +80,85 @@ struct RowSrc {
     int           M2;  // 2M
 };
 
-enum { RT_TILE, RT_SPEC };
-
 template <typename T>
 struct RArgs {
     using V2 = typename LaneOf<T>::V2;
     const T       *vin;
     T             *vout;
-    const int64_t *tile_start;  // first output row of each tile
-    const int32_t *tile_block;
-    const int64_t *blk_start;
-    const int32_t *blk_len;
-    const int32_t *blk_spec;
+    const mdp_rtile *tiles;
     const T       *H;       // [n_spec][M1][16][L/16]: spectrum / M in the order of the row kernel's registers
     const V2      *tw1;     // [R][256]: W_L^(q (k + a)) when M1 = 1, W_L^(q k) otherwise
     const V2      *tw2;     // [16][16]: W_256^(c k)
     const V2      *wa, *wb; // M1 > 1: W_M^(j2 (k1 + a)) = wa[k1][j2 >> 6] wb[k1][j2 & 63]
     const double  *means;   // [ncols][nb]
     REnt<typename LaneOf<T>::Tag> *Y;  // scratch: [item of this launch][M1][L]
-    int64_t        n_tiles, units;     // tiles; units of LaneOf::N tiles of a column of the batch
-    int64_t        item0;              // first item (column, unit) of this launch
+    int64_t        n_tiles;
+    int64_t        item0;              // first item (column of the batch, tile) of this launch
     int64_t        col_stride;
     const int     *active;  // [ncols] or nullptr
-    int            lambda, nb, E, log_m1;
+    int            lambda, nb, log_m1;
     // spectra (RT_SPEC, FP64): rows of the band and where the values go
     const double  *Trows;   // [n_spec][lambda]
     float         *H32;
     double        *H64;
 };
 
+// the tile of an item; false when its column is not to be applied
 template <typename T>
-__device__ __forceinline__ bool lanes_of(const RArgs<T> &a, int64_t item, Lane<T> (&ln)[LaneOf<T>::N],
-                                         int (&spec)[LaneOf<T>::N]) {
-    const uint32_t col = item < a.units ? 0u : (uint32_t) item / (uint32_t) a.units;
-    const int64_t  unit = item - col * a.units;
+__device__ __forceinline__ bool tile_of(const RArgs<T> &a, int64_t item, Tile<T> &tl, int &spec) {
+    const uint32_t col = item < a.n_tiles ? 0u : (uint32_t) item / (uint32_t) a.n_tiles;
+    const int64_t  tile = item - col * a.n_tiles;
     if (a.active && !a.active[col]) return false;
-#pragma unroll
-    for (int l = 0; l < LaneOf<T>::N; l++) {
-        const int64_t tile = unit * LaneOf<T>::N + l;
-        if (tile >= a.n_tiles) {
-            ln[l] = Lane<T>{a.vin, a.vout, 0, 0, 0, (T) 0};
-            spec[l] = spec[0];
-            continue;
-        }
-        const int     blk = a.tile_block[tile];
-        const int64_t bs = a.blk_start[blk] + col * a.col_stride;
-        const int     t0 = (int) (a.tile_start[tile] - a.blk_start[blk]);
-        ln[l].in = a.vin + bs;
-        ln[l].out = a.vout + bs;
-        ln[l].o = t0 - (a.lambda - 1);
-        ln[l].len = a.blk_len[blk];
-        ln[l].e = min(a.E, ln[l].len - t0);
-        ln[l].mu = a.means ? (T) a.means[col * a.nb + blk] : (T) 0;
-        spec[l] = a.blk_spec[blk];
-    }
+    const int4 d0 = __ldg(reinterpret_cast<const int4 *>(a.tiles + tile)), d1 = __ldg(reinterpret_cast<const int4 *>(a.tiles + tile) + 1);
+    const int64_t bs = (int64_t) (((uint64_t) (uint32_t) d0.y << 32) | (uint32_t) d0.x) + col * a.col_stride;
+    tl.in = a.vin + bs;
+    tl.out = a.vout + bs;
+    tl.o = d0.z;
+    tl.len = d0.w;
+    tl.e = d1.x;
+    spec = d1.y;
+    tl.mu = a.means ? (T) a.means[col * a.nb + d1.z] : (T) 0;
     return true;
 }
 
+__device__ __forceinline__ float ld_stream(const float *p) {  // read once: not kept in L1
+    float v;
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_stream(const double *p) {
+    double v;
+    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 // sample n of the window, less the block mean; zero outside the block
 template <typename T>
-__device__ __forceinline__ T sample(const Lane<T> &ln, int n) {
-    const int i = ln.o + n;
-    return (unsigned) i < (unsigned) ln.len ? __ldg(ln.in + i) - ln.mu : (T) 0;
+__device__ __forceinline__ T sample(const Tile<T> &tl, int n) {
+    const int i = tl.o + n;
+    return (unsigned) i < (unsigned) tl.len ? ld_stream(tl.in + i) - tl.mu : (T) 0;
 }
-__device__ __forceinline__ Pr<float> samples(const Lane<float> (&ln)[2], int n) { return pmk(sample(ln[0], n), sample(ln[1], n)); }
-__device__ __forceinline__ Pr<mono64> samples(const Lane<double> (&ln)[1], int n) { return Pr<mono64>{sample(ln[0], n)}; }
-__device__ __forceinline__ Pr<mono64> samples(const RowSrc &r, int n) {
-    return Pr<mono64>{n < r.lambda ? __ldg(r.T + n) : (r.M2 - n < r.lambda ? -__ldg(r.T + (r.M2 - n)) : 0.0)};
-}
-
+// the same of a window inside its block: point j0 + n, n known at compile time
 template <typename T>
-__device__ __forceinline__ void put(const Lane<T> &ln, int halo, int n, T v) {
-    if ((unsigned) (n - halo) < (unsigned) ln.e) ln.out[ln.o + n] = v;
+__device__ __forceinline__ T sample_in(const Tile<T> &tl, int j0, int n) {
+    return ld_stream(tl.in + (tl.o + j0) + n) - tl.mu;
 }
-__device__ __forceinline__ void put_all(const Lane<float> (&ln)[2], int halo, int n, Pr<float> v) {
-    put(ln[0], halo, n, plo(v));
-    put(ln[1], halo, n, phi(v));
+__device__ __forceinline__ double sample(const RowSrc &r, int n) {
+    return n < r.lambda ? __ldg(r.T + n) : (r.M2 - n < r.lambda ? -__ldg(r.T + (r.M2 - n)) : 0.0);
 }
-__device__ __forceinline__ void put_all(const Lane<double> (&ln)[1], int halo, int n, Pr<mono64> v) { put(ln[0], halo, n, v.v); }
+template <typename T>
+__device__ __forceinline__ void put(const Tile<T> &tl, int halo, int n, T v) {
+    if ((unsigned) (n - halo) < (unsigned) tl.e) tl.out[tl.o + n] = v;
+}
+template <typename T>
+__device__ __forceinline__ CP<typename LaneOf<T>::Tag> point(T x, T y) {
+    using G = typename LaneOf<T>::Tag;
+    return CP<G>{Pr<G>{x}, Pr<G>{y}};
+}
 
-// v * w, the same w on every lane
-__device__ __forceinline__ CP<float> tmul(CP<float> v, float2 w) {
-    const Pr<float> wx = pdup(w.x), wy = pdup(w.y), ny = pdup(-w.y);
-    return {pfma(v.y, ny, pmul(v.x, wx)), pfma(v.y, wx, pmul(v.x, wy))};
-}
-__device__ __forceinline__ CP<mono64> tmul(CP<mono64> v, double2 w) {
-    return {Pr<mono64>{fma(-v.y.v, w.y, v.x.v * w.x)}, Pr<mono64>{fma(v.y.v, w.x, v.x.v * w.y)}};
+// v * w
+template <typename G, typename V2>
+__device__ __forceinline__ CP<G> tmul(CP<G> v, V2 w) {
+    return {pfma(Pr<G>{-v.y.v}, Pr<G>{w.y}, pmul(v.x, Pr<G>{w.x})), pfma(v.y, Pr<G>{w.x}, pmul(v.x, Pr<G>{w.y}))};
 }
 __device__ __forceinline__ float2 wmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ double2 wmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
@@ -199,7 +193,18 @@ template <typename G> __device__ __forceinline__ CP<G> get(const REnt<G> *p) {
     const REnt<G> e = *p;
     return {e.x, e.y};
 }
-template <typename G> __device__ __forceinline__ CP<G> swapped(CP<G> v) { return {v.y, v.x}; }
+// from L2, where other CTAs wrote it
+__device__ __forceinline__ CP<mono32> get_l2(const REnt<mono32> *p) {
+    const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+    return {Pr<mono32>{v.x}, Pr<mono32>{v.y}};
+}
+__device__ __forceinline__ CP<mono64> get_l2(const REnt<mono64> *p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+    return {Pr<mono64>{v.x}, Pr<mono64>{v.y}};
+}
+
+// CTAs of 256 threads an SM: four FP32 ones (64 registers a thread: 16 points take 32), two FP64 ones
+template <typename T> constexpr int rt_ctas() { return sizeof(T) == 4 ? 4 : 2; }
 
 // ------------------------------------------------------------------ rows
 // Row of L = R 256 points, L/16 threads, 16 points a thread in every pass.
@@ -208,225 +213,304 @@ template <typename G> __device__ __forceinline__ CP<G> swapped(CP<G> v) { return
 //   pass 3  over c, thread (k_a, k_b): bins k_a + R (k_b + 16 k_c), k_c = register
 // then the product and the same passes from the other end.  Bound: the FP and
 // shared-memory pipes (4 exchanges of 32 bytes an entry).
-template <typename T, int R, bool ONE, int SRC>
-__global__ void __launch_bounds__(16 * R, R == 16 ? 2 : 32 / R) rt_rows_kernel(RArgs<T> a) {
-    using G = typename LaneOf<T>::Tag;
-    constexpr int LN = LaneOf<T>::N, L = 256 * R, NT = 16 * R, S = 16 / R;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    REnt<G> *s = reinterpret_cast<REnt<G> *>(smem_raw);
-    const int     t = threadIdx.x;
-    const int     log_m1 = ONE ? 0 : a.log_m1;
-    const int64_t li = blockIdx.x >> log_m1;  // item of this launch
-    const int     k1 = (int) blockIdx.x & ((1 << log_m1) - 1);
-    const int     M = L << log_m1;
-    Lane<T>       ln[LN];
-    int           spec[LN];
-    RowSrc        rs{};
-    if constexpr (SRC == RT_SPEC) {
-        rs = RowSrc{a.Trows + (a.item0 + li) * a.lambda, a.lambda, 2 * M};
-    } else {
-        if (!lanes_of(a, a.item0 + li, ln, spec)) return;
-    }
-    REnt<G> *Y = ONE ? nullptr : a.Y + (int64_t) blockIdx.x * L;
 
-    CP<G> u[16];
-    // pass 1
+// passes 1 to 3 of a row: in(n) gives point n; u[rev(k)] = bin of register k.  ONE: quarter shift
+template <typename T, int R, bool ONE, typename In>
+__device__ __forceinline__ void row_forward(REnt<typename LaneOf<T>::Tag> *s, const typename LaneOf<T>::V2 *tw1,
+                                            const typename LaneOf<T>::V2 *tw2, In in,
+                                            CP<typename LaneOf<T>::Tag> (&u)[16]) {
+    using G = typename LaneOf<T>::Tag;
+    constexpr int NT = 16 * R, S = 16 / R;
+    const int     t = threadIdx.x, c = t & 15, kh = t >> 4;
 #pragma unroll
     for (int j = 0; j < S; j++) {
         const int q = t + NT * j;
         CP<G>     v[R];
 #pragma unroll
-        for (int i = 0; i < R; i++) {
-            const int n = 256 * i + q;
-            if constexpr (!ONE) v[i] = get(Y + n);
-            else if constexpr (SRC == RT_SPEC) v[i] = CP<G>{samples(rs, n), samples(rs, n + M)};
-            else v[i] = CP<G>{samples(ln, n), samples(ln, n + M)};
-        }
+        for (int i = 0; i < R; i++) v[i] = in(256 * i + q);
         if constexpr (ONE) quarter_shift<G, R>(v);
         dif_reg<G, R>(v);
 #pragma unroll
         for (int k = 0; k < R; k++) {
             CP<G> w = v[rev_bits_c(k, ilog2_c(R))];
-            if (ONE || k > 0) w = tmul(w, __ldg(a.tw1 + k * 256 + q));
+            if (ONE || k > 0) w = tmul(w, __ldg(tw1 + k * 256 + q));
             s[rt_pos(k * 256 + q)] = REnt<G>{w.x, w.y};
         }
     }
     __syncthreads();
-    // pass 2
-    const int c = t & 15, kh = t >> 4;  // also pass 3: (k_a, k_b) = (kh, c)
 #pragma unroll
     for (int i = 0; i < 16; i++) u[i] = get(s + rt_pos(kh * 256 + 16 * i + c));
     dif_reg<G, 16>(u);
 #pragma unroll
     for (int k = 0; k < 16; k++) {
         CP<G> w = u[rev_bits_c(k, 4)];
-        if (k > 0) w = tmul(w, __ldg(a.tw2 + k * 16 + c));
+        if (k > 0) w = tmul(w, __ldg(tw2 + k * 16 + c));
         s[rt_pos(kh * 256 + 16 * k + c)] = REnt<G>{w.x, w.y};
     }
     __syncthreads();
-    // pass 3, the product, pass 3 back
 #pragma unroll
-    for (int i = 0; i < 16; i++) u[i] = get(s + rt_pos(kh * 256 + 16 * c + i));
+    for (int i = 0; i < 16; i++) u[i] = get(s + rt_pos(kh * 256 + 16 * c + i));  // (k_a, k_b) = (kh, c)
     dif_reg<G, 16>(u);
-    if constexpr (SRC == RT_SPEC) {
-        const int64_t at = (((a.item0 + li) << log_m1) + k1) * L + t;
-        const double  sc = 1.0 / (double) M;
+}
+
+// the passes back from z[k] (register k, parts exchanged); out(n, v) takes point n
+template <typename T, int R, bool ONE, typename Out>
+__device__ __forceinline__ void row_back(REnt<typename LaneOf<T>::Tag> *s, const typename LaneOf<T>::V2 *tw1,
+                                         const typename LaneOf<T>::V2 *tw2, CP<typename LaneOf<T>::Tag> (&z)[16],
+                                         Out out) {
+    using G = typename LaneOf<T>::Tag;
+    constexpr int NT = 16 * R, S = 16 / R;
+    const int     t = threadIdx.x, c = t & 15, kh = t >> 4;
+    dif_reg<G, 16>(z);
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const double h = u[rev_bits_c(k, 4)].x.v * sc;
-            if (a.H32) a.H32[at + k * NT] = (float) h;
-            else a.H64[at + k * NT] = h;
-        }
-        return;
-    } else {
-        CP<G>    z[16];
-        const T *h0 = a.H + (((int64_t) spec[0] << log_m1) + k1) * L + t;
+    for (int i = 0; i < 16; i++) {
+        CP<G> w = z[rev_bits_c(i, 4)];
+        if (i > 0) w = tmul(w, __ldg(tw2 + i * 16 + c));  // W_256^(c k_b), symmetric
+        s[rt_pos(kh * 256 + 16 * c + i)] = REnt<G>{w.x, w.y};
+    }
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const CP<G> w = u[rev_bits_c(k, 4)];
-            Pr<G>       h;
-            if constexpr (LN == 2) {
-                const T *h1 = a.H + (((int64_t) spec[LN - 1] << log_m1) + k1) * L + t;
-                h = pmk(__ldg(h0 + k * NT), __ldg(h1 + k * NT));
-            } else {
-                h = Pr<G>{__ldg(h0 + k * NT)};
-            }
-            z[k] = CP<G>{pmul(w.y, h), pmul(w.x, h)};  // real and imaginary parts exchanged from here on
-        }
-        dif_reg<G, 16>(z);
+    for (int k = 0; k < 16; k++) z[k] = get(s + rt_pos(kh * 256 + 16 * k + c));
+    dif_reg<G, 16>(z);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            CP<G> w = z[rev_bits_c(i, 4)];
-            if (i > 0) w = tmul(w, __ldg(a.tw2 + i * 16 + c));  // W_256^(c k_b), symmetric
-            s[rt_pos(kh * 256 + 16 * c + i)] = REnt<G>{w.x, w.y};
-        }
-        __syncthreads();
-        // pass 2 back
+    for (int i = 0; i < 16; i++) {
+        const CP<G> w = tmul(z[rev_bits_c(i, 4)], __ldg(tw1 + kh * 256 + 16 * i + c));
+        s[rt_pos(kh * 256 + 16 * i + c)] = REnt<G>{w.x, w.y};
+    }
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; k++) z[k] = get(s + rt_pos(kh * 256 + 16 * k + c));
-        dif_reg<G, 16>(z);
+    for (int j = 0; j < S; j++) {
+        const int q = t + NT * j;
+        CP<G>     v[R], y[R];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const CP<G> w = tmul(z[rev_bits_c(i, 4)], __ldg(a.tw1 + kh * 256 + 16 * i + c));
-            s[rt_pos(kh * 256 + 16 * i + c)] = REnt<G>{w.x, w.y};
-        }
-        __syncthreads();
-        // pass 1 back
+        for (int k = 0; k < R; k++) v[k] = get(s + rt_pos(k * 256 + q));
+        dif_reg<G, R>(v);
 #pragma unroll
-        for (int j = 0; j < S; j++) {
-            const int q = t + NT * j;
-            CP<G>     v[R], y[R];
+        for (int i = 0; i < R; i++) y[i] = v[rev_bits_c(i, ilog2_c(R))];
+        if constexpr (ONE) quarter_shift<G, R>(y);
 #pragma unroll
-            for (int k = 0; k < R; k++) v[k] = get(s + rt_pos(k * 256 + q));
-            dif_reg<G, R>(v);
+        for (int i = 0; i < R; i++) out(256 * i + q, y[i]);
+    }
+}
+
+// z[k] = u[rev(k)] H, real and imaginary parts exchanged
+template <typename T, typename G>
+__device__ __forceinline__ void row_product(const CP<G> (&u)[16], const T *h, int nt, CP<G> (&z)[16]) {
 #pragma unroll
-            for (int i = 0; i < R; i++) y[i] = v[rev_bits_c(i, ilog2_c(R))];
-            if constexpr (ONE) quarter_shift<G, R>(y);
+    for (int k = 0; k < 16; k++) {
+        const CP<G> w = u[rev_bits_c(k, 4)];
+        const Pr<G> hk{ld_stream(h + k * nt)};
+        z[k] = CP<G>{pmul(w.y, hk), pmul(w.x, hk)};
+    }
+}
+
+// tiles of one row (M = L): samples in, outputs out
+template <typename T, int R>
+__global__ void __launch_bounds__(16 * R, rt_ctas<T>() * 16 / R) rt_one_kernel(RArgs<T> a) {
+    using G = typename LaneOf<T>::Tag;
+    constexpr int M = 256 * R, NT = 16 * R;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    REnt<G> *s = reinterpret_cast<REnt<G> *>(smem_raw);
+    Tile<T>  tl;
+    int      spec;
+    if (!tile_of(a, a.item0 + blockIdx.x, tl, spec)) return;
+    CP<G>     u[16], z[16];
+    const int halo = a.lambda - 1;
+    row_forward<T, R, true>(s, a.tw1, a.tw2, [&](int n) { return point(sample(tl, n), sample(tl, n + M)); }, u);
+    row_product(u, a.H + (int64_t) spec * M + threadIdx.x, NT, z);
+    row_back<T, R, true>(s, a.tw1, a.tw2, z, [&](int n, CP<G> y) {
+        put(tl, halo, n, y.y.v);
+        put(tl, halo, n + M, y.x.v);
+    });
+}
+
+// the spectra / M of rows of the band (FP64): one-row tiles (ONE) or the rows after the columns
+template <int R, bool ONE>
+__global__ void __launch_bounds__(16 * R, R == 16 ? 2 : 32 / R) rt_spec_rows_kernel(RArgs<double> a) {
+    constexpr int L = 256 * R, NT = 16 * R;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    REnt<mono64> *s = reinterpret_cast<REnt<mono64> *>(smem_raw);
+    const int     M = L << a.log_m1;
+    const RowSrc  rs{a.Trows + (a.item0 + blockIdx.x) * a.lambda, a.lambda, 2 * M};
+    REnt<mono64> *Y = a.Y + (int64_t) blockIdx.x * L;
+    CP<mono64>    u[16];
+    row_forward<double, R, ONE>(s, a.tw1, a.tw2, [&](int n) {
+        if constexpr (ONE) return point(sample(rs, n), sample(rs, n + M));
+        else return get(Y + n);
+    }, u);
+    const int64_t at = ((a.item0 << a.log_m1) + blockIdx.x) * L + threadIdx.x;
+    const double  sc = 1.0 / (double) M;
 #pragma unroll
-            for (int i = 0; i < R; i++) {
-                const int n = 256 * i + q;
-                if constexpr (ONE) {
-                    put_all(ln, a.lambda - 1, n, y[i].y);
-                    put_all(ln, a.lambda - 1, n + M, y[i].x);
-                } else {
-                    Y[n] = REnt<G>{y[i].x, y[i].y};
-                }
-            }
-        }
+    for (int k = 0; k < 16; k++) {
+        const double h = u[rev_bits_c(k, 4)].x.v * sc;
+        if (a.H32) a.H32[at + k * NT] = (float) h;
+        else a.H64[at + k * NT] = h;
     }
 }
 
 // ------------------------------------------------------------------ columns
 // M1-point transforms over j1 of the columns j2, one thread a column, 16 points a
-// thread; L = 4096.  Bound: memory (samples in, scratch out, and back).
-template <typename T, int M1, bool INV, int SRC>
-__global__ void __launch_bounds__(256, 2) rt_cols_kernel(RArgs<T> a) {
+// thread: part p of M1 covers columns p (4096/M1) on; L = 4096.
+template <typename T, int M1, typename In>
+__device__ __forceinline__ void cols_forward(const RArgs<T> &a, int part, REnt<typename LaneOf<T>::Tag> *Y, In in) {
     using G = typename LaneOf<T>::Tag;
-    constexpr int LN = LaneOf<T>::N, L = 4096, M = M1 * L, S = 16 / M1;
-    const int64_t li = blockIdx.x / (unsigned) M1;
-    const int     j0 = (int) (blockIdx.x % M1) * (256 * S) + threadIdx.x;
-    Lane<T>       ln[LN];
-    int           spec[LN];
-    RowSrc        rs{};
-    if constexpr (SRC == RT_SPEC) {
-        rs = RowSrc{a.Trows + (a.item0 + li) * a.lambda, a.lambda, 2 * M};
-    } else {
-        if (!lanes_of(a, a.item0 + li, ln, spec)) return;
-    }
-    REnt<G> *Y = a.Y + li * M;
-    CP<G>    v[S][M1];
-    if constexpr (!INV) {
+    constexpr int L = 4096, S = 16 / M1;
+    const int     j0 = part * (256 * S) + (int) threadIdx.x;
+    CP<G>         v[S][M1];
 #pragma unroll
-        for (int j = 0; j < S; j++)
+    for (int j = 0; j < S; j++)
 #pragma unroll
-            for (int i = 0; i < M1; i++) {
-                const int n = L * i + j0 + 256 * j;
-                if constexpr (SRC == RT_SPEC) v[j][i] = CP<G>{samples(rs, n), samples(rs, n + M)};
-                else v[j][i] = CP<G>{samples(ln, n), samples(ln, n + M)};
-            }
-    } else {
-#pragma unroll
-        for (int j = 0; j < S; j++)
-#pragma unroll
-            for (int k = 0; k < M1; k++) v[j][k] = get(Y + k * L + j0 + 256 * j);
-    }
+        for (int i = 0; i < M1; i++) v[j][i] = in(j0, L * i + 256 * j);
 #pragma unroll
     for (int j = 0; j < S; j++) {
         const int j2 = j0 + 256 * j;
-        if constexpr (!INV) {
-            quarter_shift<G, M1>(v[j]);
-            dif_reg<G, M1>(v[j]);
+        quarter_shift<G, M1>(v[j]);
+        dif_reg<G, M1>(v[j]);
 #pragma unroll
-            for (int k = 0; k < M1; k++) {
-                const CP<G> w = tmul(v[j][rev_bits_c(k, ilog2_c(M1))],
-                                     wmul(__ldg(a.wa + k * 64 + (j2 >> 6)), __ldg(a.wb + k * 64 + (j2 & 63))));
-                Y[k * L + j2] = REnt<G>{w.x, w.y};
-            }
-        } else {  // real and imaginary parts exchanged
-#pragma unroll
-            for (int k = 0; k < M1; k++)
-                v[j][k] = tmul(v[j][k], wmul(__ldg(a.wa + k * 64 + (j2 >> 6)), __ldg(a.wb + k * 64 + (j2 & 63))));
-            dif_reg<G, M1>(v[j]);
-            CP<G> y[M1];
-#pragma unroll
-            for (int i = 0; i < M1; i++) y[i] = v[j][rev_bits_c(i, ilog2_c(M1))];
-            quarter_shift<G, M1>(y);
-#pragma unroll
-            for (int i = 0; i < M1; i++) {
-                put_all(ln, a.lambda - 1, L * i + j2, y[i].y);
-                put_all(ln, a.lambda - 1, L * i + j2 + M, y[i].x);
-            }
+        for (int k = 0; k < M1; k++) {
+            const CP<G> w = tmul(v[j][rev_bits_c(k, ilog2_c(M1))],
+                                 wmul(__ldg(a.wa + k * 64 + (j2 >> 6)), __ldg(a.wb + k * 64 + (j2 & 63))));
+            Y[k * L + j2] = REnt<G>{w.x, w.y};
         }
     }
+}
+
+// and back, from rows whose parts are exchanged
+template <typename T, int M1>
+__device__ __forceinline__ void cols_back(const RArgs<T> &a, int part, const REnt<typename LaneOf<T>::Tag> *Y,
+                                          const Tile<T> &tl) {
+    using G = typename LaneOf<T>::Tag;
+    constexpr int L = 4096, M = M1 * L, S = 16 / M1;
+    const int     j0 = part * (256 * S) + (int) threadIdx.x, halo = a.lambda - 1;
+    CP<G>         v[S][M1];
+#pragma unroll
+    for (int j = 0; j < S; j++)
+#pragma unroll
+        for (int k = 0; k < M1; k++) v[j][k] = get_l2(Y + k * L + j0 + 256 * j);
+#pragma unroll
+    for (int j = 0; j < S; j++) {
+        const int j2 = j0 + 256 * j;
+#pragma unroll
+        for (int k = 0; k < M1; k++)
+            v[j][k] = tmul(v[j][k], wmul(__ldg(a.wa + k * 64 + (j2 >> 6)), __ldg(a.wb + k * 64 + (j2 & 63))));
+        dif_reg<G, M1>(v[j]);
+        CP<G> y[M1];
+#pragma unroll
+        for (int i = 0; i < M1; i++) y[i] = v[j][rev_bits_c(i, ilog2_c(M1))];
+        quarter_shift<G, M1>(y);
+#pragma unroll
+        for (int i = 0; i < M1; i++) {
+            put(tl, halo, L * i + j2, y[i].y.v);
+            put(tl, halo, L * i + j2 + M, y[i].x.v);
+        }
+    }
+}
+
+template <int M1>
+__global__ void __launch_bounds__(256, 2) rt_spec_cols_kernel(RArgs<double> a) {
+    constexpr int M = M1 * 4096;
+    const int64_t li = blockIdx.x / (unsigned) M1;
+    const RowSrc  rs{a.Trows + (a.item0 + li) * a.lambda, a.lambda, 2 * M};
+    cols_forward<double, M1>(a, (int) (blockIdx.x % M1), a.Y + li * M,
+                             [&](int j0, int n) { return point(sample(rs, j0 + n), sample(rs, j0 + n + M)); });
+}
+
+template <typename T, int M1>
+__global__ void __launch_bounds__(256, rt_ctas<T>()) rt_cols_kernel(RArgs<T> a) {
+    constexpr int M = M1 * 4096;
+    const int     li = blockIdx.x / (unsigned) M1, part = blockIdx.x % (unsigned) M1;
+    Tile<T>       tl;
+    int           spec;
+    if (!tile_of(a, a.item0 + li, tl, spec)) return;
+    auto *Y = a.Y + (int64_t) li * M;
+    if (tl.o >= 0 && tl.o + 2 * M <= tl.len)
+        cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample_in(tl, j0, n), sample_in(tl, j0, n + M)); });
+    else
+        cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample(tl, j0 + n), sample(tl, j0 + n + M)); });
+}
+template <typename T, int M1>
+__global__ void __launch_bounds__(256, rt_ctas<T>()) rt_cols_back_kernel(RArgs<T> a) {
+    constexpr int M = M1 * 4096;
+    const int     li = blockIdx.x / (unsigned) M1, part = blockIdx.x % (unsigned) M1;
+    Tile<T>       tl;
+    int           spec;
+    if (!tile_of(a, a.item0 + li, tl, spec)) return;
+    cols_back<T, M1>(a, part, a.Y + (int64_t) li * M, tl);
+}
+template <typename T>
+__global__ void __launch_bounds__(256, rt_ctas<T>()) rt_rows_kernel(RArgs<T> a) {
+    using G = typename LaneOf<T>::Tag;
+    constexpr int L = 4096;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    REnt<G>  *s = reinterpret_cast<REnt<G> *>(smem_raw);
+    const int li = blockIdx.x >> a.log_m1, part = blockIdx.x & ((1 << a.log_m1) - 1);
+    Tile<T>   tl;
+    int       spec;
+    if (!tile_of(a, a.item0 + li, tl, spec)) return;
+    REnt<G> *row = a.Y + (int64_t) blockIdx.x * L;
+    CP<G>    u[16], z[16];
+    row_forward<T, 16, false>(s, a.tw1, a.tw2, [&](int n) { return get_l2(row + n); }, u);
+    row_product(u, a.H + (((int64_t) spec << a.log_m1) + part) * L + threadIdx.x, 256, z);
+    row_back<T, 16, false>(s, a.tw1, a.tw2, z, [&](int n, CP<G> y) { row[n] = REnt<G>{y.x, y.y}; });
 }
 
 // ------------------------------------------------------------------ host side
-// items (tiles of FP64, pairs of tiles of FP32) whose columns, rows and columns back
-// are launched together: their scratch stays in L2 between the three kernels
-#ifndef RT_GROUP_BYTES
-#define RT_GROUP_BYTES (int64_t(64) << 20)
-#endif
-
-template <typename T> size_t rows_smem(int L) { return 16 * (size_t) rt_entries(L); }
-
-template <typename T, bool ONE, int SRC>
-const void *rows_fn(int L) {
-    if constexpr (ONE) {
-        switch (L) {
-            case 512: return (const void *) rt_rows_kernel<T, 2, true, SRC>;
-            case 1024: return (const void *) rt_rows_kernel<T, 4, true, SRC>;
-            case 2048: return (const void *) rt_rows_kernel<T, 8, true, SRC>;
-        }
-    }
-    return L == 4096 ? (const void *) rt_rows_kernel<T, 16, ONE, SRC> : nullptr;
+template <typename T> size_t rows_smem(int L) { return 2 * sizeof(T) * (size_t) rt_entries(L); }
+// Items whose columns, rows and columns back are launched together, so that their scratch
+// stays in L2 (126 MB) between the three kernels.  Groups alternate between the context's
+// stream and its side stream with a scratch half each: the last CTAs of one group's kernel
+// and the next launch share the device with the other group's.  64 x 2^20 samples, half
+// bandwidth 2^14, one stream and 64 MB -> two and 64 MB each: FP32 0.70 -> 0.645 ms, FP64 1.34
+// -> 1.20 ms (halves of 24, 32, 48 MB: 0.68, 0.66, 0.64 and 1.24, 1.21, 1.24 ms); work that fits
+// one half is cut in two from 2 x 16 MB on (8 x 2^20, 2^13, FP32: 99 -> 96 us).
+constexpr int64_t RT_HALF_BYTES = int64_t(64) << 20, RT_MIN_BYTES = int64_t(16) << 20;
+struct Groups {
+    int64_t n, per;  // how many, items in each but the last
+};
+Groups groups_of(int64_t items, int64_t item_bytes, int64_t cap) {
+    const int64_t half = std::min<int64_t>(RT_HALF_BYTES, cap / 2 >= item_bytes ? cap / 2 : cap);
+    int64_t       n = std::max<int64_t>(1, (items * item_bytes + half - 1) / half);
+    if (n == 1 && items > 1 && items * item_bytes >= 2 * RT_MIN_BYTES) n = 2;
+    const int64_t per = std::min<int64_t>((items + n - 1) / n, std::max<int64_t>(1, half / item_bytes));
+    return Groups{(items + per - 1) / per, per};
 }
-template <typename T, bool INV, int SRC>
-const void *cols_fn(int m1) {
+
+template <typename T>
+const void *one_fn(int L) {
+    switch (L) {
+        case 512: return (const void *) rt_one_kernel<T, 2>;
+        case 1024: return (const void *) rt_one_kernel<T, 4>;
+        case 2048: return (const void *) rt_one_kernel<T, 8>;
+        case 4096: return (const void *) rt_one_kernel<T, 16>;
+    }
+    return nullptr;
+}
+template <typename T, bool BACK>
+const void *cols_fn(int log_m1) {
+    switch (log_m1) {
+        case 1: return BACK ? (const void *) rt_cols_back_kernel<T, 2> : (const void *) rt_cols_kernel<T, 2>;
+        case 2: return BACK ? (const void *) rt_cols_back_kernel<T, 4> : (const void *) rt_cols_kernel<T, 4>;
+        case 3: return BACK ? (const void *) rt_cols_back_kernel<T, 8> : (const void *) rt_cols_kernel<T, 8>;
+        case 4: return BACK ? (const void *) rt_cols_back_kernel<T, 16> : (const void *) rt_cols_kernel<T, 16>;
+    }
+    return nullptr;
+}
+const void *spec_rows_fn(int m1, int L) {
+    if (m1 > 1) return (const void *) rt_spec_rows_kernel<16, false>;
+    switch (L) {
+        case 512: return (const void *) rt_spec_rows_kernel<2, true>;
+        case 1024: return (const void *) rt_spec_rows_kernel<4, true>;
+        case 2048: return (const void *) rt_spec_rows_kernel<8, true>;
+        case 4096: return (const void *) rt_spec_rows_kernel<16, true>;
+    }
+    return nullptr;
+}
+const void *spec_cols_fn(int m1) {
     switch (m1) {
-        case 2: return (const void *) rt_cols_kernel<T, 2, INV, SRC>;
-        case 4: return (const void *) rt_cols_kernel<T, 4, INV, SRC>;
-        case 8: return (const void *) rt_cols_kernel<T, 8, INV, SRC>;
-        case 16: return (const void *) rt_cols_kernel<T, 16, INV, SRC>;
+        case 2: return (const void *) rt_spec_cols_kernel<2>;
+        case 4: return (const void *) rt_spec_cols_kernel<4>;
+        case 8: return (const void *) rt_spec_cols_kernel<8>;
+        case 16: return (const void *) rt_spec_cols_kernel<16>;
     }
     return nullptr;
 }
@@ -470,9 +554,6 @@ int build_tables(int m1, int L, DevBuf &buf, const V2 **tw1, const V2 **tw2, con
     return MDP_OK;
 }
 
-template <typename T>
-int64_t group_items(int64_t M) { return std::max<int64_t>(1, RT_GROUP_BYTES / (16 * M)); }
-
 }  // namespace
 
 bool rtile_shape(int log_m1, int log_m2) {
@@ -486,18 +567,33 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
     using V2 = typename LaneOf<T>::V2;
     const int m1 = 1 << P.log_m1, L = 1 << P.log_m2, M = m1 * L;
     if (!rtile_shape(P.log_m1, P.log_m2)) return MDP_EUNSUPPORTED;
+    // where each tile's window lies, in one 32-byte record (a chain of loads through the tile, its
+    // block and the block's place would be on every CTA's path)
+    {
+        std::vector<mdp_rtile> tiles;
+        const int64_t          E = P.fft_n - 2LL * (N->lambda - 1);
+        for (int b = 0; b < N->nb; b++)
+            for (int64_t o = 0; o < N->h_n[b]; o += E)
+                tiles.push_back(mdp_rtile{N->h_idv[b], (int32_t) (o - (N->lambda - 1)), N->h_n[b],
+                                          (int32_t) std::min<int64_t>(E, N->h_n[b] - o), N->h_spec.empty() ? 0 : N->h_spec[b],
+                                          b, 0});
+        MDP_TRY(P.tile_start.alloc(sizeof(mdp_rtile) * std::max<size_t>(tiles.size(), 1)));
+        if (!tiles.empty())
+            MDP_CUDA(cudaMemcpy(P.tile_start.p, tiles.data(), sizeof(mdp_rtile) * tiles.size(), cudaMemcpyHostToDevice));
+    }
     const V2 *p[4];
     MDP_TRY(build_tables<V2>(m1, L, P.ltw, &p[0], &p[1], &p[2], &p[3]));
-    const int64_t units = (P.n_tiles + LaneOf<T>::N - 1) / LaneOf<T>::N;
     if (m1 > 1) {
         // FP32 plans also run column batches of up to 8 columns
-        const int64_t items = std::min(group_items<T>(M), std::max<int64_t>(1, units * (sizeof(T) == 4 ? 8 : 1)));
-        MDP_TRY(P.scratch.alloc(16 * (size_t) items * M));
+        const int64_t items = std::max<int64_t>(1, P.n_tiles * (sizeof(T) == 4 ? 8 : 1));
+        const int64_t most = std::max<int64_t>(2, 2 * RT_HALF_BYTES / (int64_t) (2 * sizeof(T) * M));
+        MDP_TRY(P.scratch.alloc(2 * sizeof(T) * (size_t) M * (size_t) std::min(items, most)));
+        MDP_CUDA(cudaFuncSetAttribute((const void *) rt_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<T>(L)));
+    } else {
+        MDP_CUDA(cudaFuncSetAttribute(one_fn<T>(L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<T>(L)));
     }
     const size_t nh = (size_t) std::max(N->n_spec, 1) * M;
     MDP_TRY(P.spectra.alloc(sizeof(T) * nh));
-    const void *fr = m1 == 1 ? rows_fn<T, true, RT_TILE>(L) : rows_fn<T, false, RT_TILE>(L);
-    MDP_CUDA(cudaFuncSetAttribute(fr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<T>(L)));
     if (!spectra) {
         MDP_CUDA(cudaMemset(P.spectra.p, 0, sizeof(T) * nh));
         return MDP_OK;
@@ -508,7 +604,7 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
     MDP_TRY(rows.alloc(sizeof(double) * N->h_Tuniq.size()));
     MDP_CUDA(cudaMemcpyAsync(rows.p, N->h_Tuniq.data(), sizeof(double) * N->h_Tuniq.size(), cudaMemcpyHostToDevice,
                              ctx->stream));
-    const int64_t per = m1 > 1 ? std::min<int64_t>(N->n_spec, group_items<double>(M)) : N->n_spec;
+    const int64_t per = m1 > 1 ? std::min<int64_t>(N->n_spec, 64) : N->n_spec;
     if (m1 > 1) MDP_TRY(Y.alloc(16 * (size_t) per * M));
     a.Trows = rows.as<double>();
     a.lambda = N->lambda;
@@ -516,15 +612,14 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
     a.Y = Y.as<REnt<mono64>>();
     if (sizeof(T) == 4) a.H32 = P.spectra.as<float>();
     else a.H64 = P.spectra.as<double>();
-    const void *fs = m1 == 1 ? rows_fn<double, true, RT_SPEC>(L) : rows_fn<double, false, RT_SPEC>(L);
+    const void *fs = spec_rows_fn(m1, L);
     MDP_CUDA(cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<double>(L)));
     for (int64_t i = 0; i < N->n_spec; i += per) {
         const int64_t n = std::min<int64_t>(per, N->n_spec - i);
         a.item0 = i;
         void *args[] = {&a};
         if (m1 > 1) {
-            MDP_CUDA(cudaLaunchKernel(cols_fn<double, false, RT_SPEC>(m1), dim3((unsigned) (n * m1)), dim3(256), args, 0,
-                                      ctx->stream));
+            MDP_CUDA(cudaLaunchKernel(spec_cols_fn(m1), dim3((unsigned) (n * m1)), dim3(256), args, 0, ctx->stream));
             MDP_CHECK_LAUNCH(ctx);
         }
         MDP_CUDA(cudaLaunchKernel(fs, dim3((unsigned) (n * m1)), dim3(L / 16), args, rows_smem<double>(L), ctx->stream));
@@ -542,11 +637,7 @@ int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, c
     RArgs<T>  a{};
     a.vin = d_in;
     a.vout = d_out;
-    a.tile_start = P.tile_start.as<int64_t>();
-    a.tile_block = P.tile_block.as<int32_t>();
-    a.blk_start = N->blk_start.as<int64_t>();
-    a.blk_len = N->blk_len.as<int32_t>();
-    a.blk_spec = N->blk_spec.as<int32_t>();
+    a.tiles = P.tile_start.as<mdp_rtile>();
     a.H = P.spectra.as<T>();
     a.tw1 = P.ltw.as<V2>();
     a.tw2 = a.tw1 + L;
@@ -555,33 +646,39 @@ int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, c
     a.means = d_means;
     a.Y = P.scratch.as<REnt<typename LaneOf<T>::Tag>>();
     a.n_tiles = P.n_tiles;
-    a.units = (P.n_tiles + LaneOf<T>::N - 1) / LaneOf<T>::N;
     a.col_stride = col_stride;
     a.active = d_active;
     a.lambda = N->lambda;
     a.nb = N->nb;
-    a.E = P.fft_n - 2 * (N->lambda - 1);
     a.log_m1 = P.log_m1;
-    const int64_t items = a.units * ncols;
+    const int64_t items = P.n_tiles * ncols;
     if (items << P.log_m1 > 0x7fffffffLL) return MDP_EUNSUPPORTED;
-    const int64_t per = m1 > 1 ? (int64_t) (P.scratch.bytes / (16 * (size_t) M)) : (int64_t) 0x7fffffff;
-    const void   *fr = m1 == 1 ? rows_fn<T, true, RT_TILE>(L) : rows_fn<T, false, RT_TILE>(L);
-    for (int64_t i = 0; i < items; i += per) {
-        const int64_t n = std::min(per, items - i);
-        a.item0 = i;
-        void      *args[] = {&a};
-        const dim3 grid((unsigned) (n * m1));
-        if (m1 > 1) {
-            MDP_CUDA(cudaLaunchKernel(cols_fn<T, false, RT_TILE>(m1), grid, dim3(256), args, 0, ctx->stream));
-            MDP_CHECK_LAUNCH(ctx);
-        }
-        MDP_CUDA(cudaLaunchKernel(fr, grid, dim3(L / 16), args, rows_smem<T>(L), ctx->stream));
+    void *args[] = {&a};
+    if (m1 == 1) {
+        MDP_CUDA(cudaLaunchKernel(one_fn<T>(L), dim3((unsigned) items), dim3(L / 16), args, rows_smem<T>(L), ctx->stream));
         MDP_CHECK_LAUNCH(ctx);
-        if (m1 > 1) {
-            MDP_CUDA(cudaLaunchKernel(cols_fn<T, true, RT_TILE>(m1), grid, dim3(256), args, 0, ctx->stream));
-            MDP_CHECK_LAUNCH(ctx);
-        }
+        return MDP_OK;
     }
+    const Groups g = groups_of(items, 2 * (int64_t) sizeof(T) * M, (int64_t) P.scratch.bytes);
+    cudaStream_t st[2] = {ctx->stream, ctx->stream};
+    if (g.n > 1) {
+        MDP_TRY(mdp_side_fork(ctx));
+        st[1] = ctx->side;
+    }
+    auto *Y = a.Y;
+    for (int64_t k = 0; k < g.n; k++) {
+        const int64_t i = k * g.per;
+        const dim3    grid((unsigned) (std::min(g.per, items - i) * m1));
+        a.item0 = i;
+        a.Y = Y + (k & 1) * g.per * M;
+        MDP_CUDA(cudaLaunchKernel(cols_fn<T, false>(P.log_m1), grid, dim3(256), args, 0, st[k & 1]));
+        MDP_CHECK_LAUNCH(ctx);
+        MDP_CUDA(cudaLaunchKernel((const void *) rt_rows_kernel<T>, grid, dim3(256), args, rows_smem<T>(L), st[k & 1]));
+        MDP_CHECK_LAUNCH(ctx);
+        MDP_CUDA(cudaLaunchKernel(cols_fn<T, true>(P.log_m1), grid, dim3(256), args, 0, st[k & 1]));
+        MDP_CHECK_LAUNCH(ctx);
+    }
+    if (g.n > 1) MDP_TRY(mdp_side_join(ctx));
     return MDP_OK;
 }
 

@@ -1811,6 +1811,7 @@ extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *
             }
             spec_of[b] = found;
         }
+        N->h_spec = spec_of;
         N->n_spec = (int) uniq.size();
         N->h_Tuniq.resize((size_t) N->n_spec * lambda);
         for (int u = 0; u < N->n_spec; u++)
