@@ -116,17 +116,17 @@ struct mdp_pt_bins {
     int64_t nbins = 0;
     DevBuf  start;   // int64 [nbins+1] offsets into perm
     DevBuf  perm;    // uint32 [valid rows] sample index, grouped by bin
+    DevBuf  pix;     // uint8 [valid rows] the row's pixel inside its bin (with slices)
     // slices of the bins' lists (P^T): every bin's list cut into runs of at
-    // most slice_len rows (one run for an empty bin); a bin of one slice is
-    // written by it, the slices of a longer bin write partial maps that are
-    // then summed in slice order.  The partial buffer belongs to the pointing:
-    // two P^T of one pointing must not run at the same time.
+    // most slice_len rows (one run for an empty bin), taken by the warps of groups (CTAs) of
+    // eight: the slices of one long bin, of equal length, or eight bins of one slice.  A bin of several groups has partial maps, summed in order; they belong
+    // to the pointing: two P^T of one pointing must not run at the same time.
     int64_t nslices = 0, nmulti = 0, slice_len = 0;
     DevBuf  slice_bin;    // int32 [nslices]
     DevBuf  slice_lo;     // uint32 [nslices] first list entry
     DevBuf  slice_hi;     // uint32 [nslices] one past the last
-    DevBuf  slice_out;    // int32 [nslices] -1: the bin's map entries, else its row of `partial`
-    DevBuf  multi_bin;    // int32 [nmulti] bins of several slices
+    DevBuf  group_out;    // int32 [groups] -2: each warp's bin, -1: the group's bin, else its row of `partial`
+    DevBuf  multi_bin;    // int32 [nmulti] bins of several groups
     DevBuf  multi_first;  // int32 [nmulti] their first row of `partial`
     DevBuf  multi_n;      // int32 [nmulti] and how many
     DevBuf  partial;      // double [rows][3 bin_pix]

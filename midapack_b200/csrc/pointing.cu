@@ -638,8 +638,9 @@ __global__ void trmatvec_general_kernel(const int32_t *__restrict__ local, const
 // shared-memory copy of the bin's map.  A step whose offsets run strictly up
 // or down the lanes hits distinct pixels; in any other step the rows that hit
 // the same pixel are summed in lane order by the group's lowest lane, which
-// adds the sum.  A bin of one slice is written by that warp;
-// the slices of a longer bin write partial maps, summed in slice order by one
+// adds the sum.  A bin of one slice is written by that warp; the slices of a longer
+// bin go to CTAs of their own, PT_WARPS a CTA, whose sums are added in slice order, and
+// a bin of several CTAs gets their partial maps summed in order by one
 // thread per map entry.  The order of every addition is fixed, so the sums
 // are reproducible bit for bit, and no atomic operation touches the map.
 // Slicing keeps the work per warp bounded: small maps (few bins) still fill
@@ -687,12 +688,13 @@ __global__ void bin_offsets_kernel(uint32_t *__restrict__ count, int64_t nchunks
     }
 }
 
-// one warp per chunk: its rows in order into their bins' lists (cursor row of
-// the chunk in shared memory when it fits, else in place in global memory)
+// one warp per chunk: its rows in order into their bins' lists, with their pixels inside the
+// bin when pix is given (cursor row of the chunk in shared memory when it fits, else in place
+// in global memory)
 __global__ void __launch_bounds__(32) bin_chunk_scatter_kernel(const int32_t *__restrict__ off, int64_t m, int bin3,
                                                                int64_t chunk, int64_t nbins,
                                                                uint32_t *__restrict__ offs, uint32_t *__restrict__ perm,
-                                                               int use_smem) {
+                                                               uint8_t *__restrict__ pix, int use_smem) {
     extern __shared__ uint32_t cur_s[];
     const int64_t c = blockIdx.x;
     const int64_t r0 = c * chunk, r1 = min(m, r0 + chunk);
@@ -722,7 +724,11 @@ __global__ void __launch_bounds__(32) bin_chunk_scatter_kernel(const int32_t *__
                 cur[b] = base + (uint32_t) __popc(peers);
             }
             base = __shfl_sync(0xffffffffu, base, leader);
-            if (b >= 0) perm[base + __popc(peers & below)] = (uint32_t) t;
+            if (b >= 0) {
+                const uint32_t at = base + __popc(peers & below);
+                perm[at] = (uint32_t) t;
+                if (pix) pix[at] = (uint8_t) ((o[u] - b * bin3) / 3);
+            }
             __syncwarp();
         }
     }
@@ -732,8 +738,8 @@ __global__ void __launch_bounds__(32) bin_chunk_scatter_kernel(const int32_t *__
 // device whatever the map size, at least 512 and at most 2^16 rows each; a
 // function of the pointing alone (rows and bins), so that the sums are the
 // same on every device.  Longer slices would leave a small map's few bins to a few warps;
-// shorter ones write more partial maps (3 bin_pix doubles per slice of a bin
-// cut in several).
+// shorter ones write more partial maps (3 bin_pix doubles per PT_WARPS slices of a
+// bin cut in more).
 static int64_t pt_slice_len(int64_t m, int64_t nbins) {
     int64_t len = 512;
     while (len < (1 << 16) && m / len > (1 << 14)) len <<= 1;
@@ -775,6 +781,7 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
     uint32_t total = 0;
     MDP_TRY(mdp_exclusive_scan_u32(ctx, tot.as<uint32_t>(), start.as<uint32_t>(), nb + 1, &total));
     MDP_TRY(B->perm.alloc(4 * std::max<int64_t>(total, 1)));
+    if (slices) MDP_TRY(B->pix.alloc(std::max<int64_t>(total, 1)));
     if (nb > 0) {
         bin_offsets_kernel<<<grid_for(nb, 256, 1024), 256, 0, ctx->stream>>>(count.as<uint32_t>(), nch, nb,
                                                                              start.as<uint32_t>());
@@ -787,7 +794,7 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
             MDP_CUDA(cudaFuncSetAttribute((const void *) bin_chunk_scatter_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm));
         bin_chunk_scatter_kernel<<<(unsigned) nch, 32, use_smem ? sm : 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->m, bin3, chunk, nb, count.as<uint32_t>(), B->perm.as<uint32_t>(), use_smem);
+                A->off.as<int32_t>(), A->m, bin3, chunk, nb, count.as<uint32_t>(), B->perm.as<uint32_t>(), slices ? B->pix.as<uint8_t>() : nullptr, use_smem);
         MDP_CHECK_LAUNCH(ctx);
     }
     std::vector<uint32_t> hs(nb + 1);
@@ -799,36 +806,46 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
     MDP_CUDA(cudaMemcpy(B->start.p, hs64.data(), 8 * (nb + 1), cudaMemcpyHostToDevice));
     B->nslices = B->nmulti = 0;
     if (slices && nb > 0) {
-        const int64_t        len = pt_slice_len(A->m, nb);
-        std::vector<int32_t> sb, so, mb, mf, mn;
+        const int64_t         len = pt_slice_len(A->m, nb);
         std::vector<uint32_t> lo, hi;
-        int32_t              rows = 0;
+        std::vector<int32_t>  sb, go, mb, mf, mn;
+        int32_t               rows = 0;
+        auto slice = [&](int64_t b, int64_t l, int64_t h) {
+            sb.push_back((int32_t) b);
+            lo.push_back((uint32_t) l);
+            hi.push_back((uint32_t) h);
+        };
+        // bins of several slices: groups of PT_WARPS slices, the bin's rows spread over them evenly
+        // (whole steps of 32 rows), a group's output the bin itself or a partial map
         for (int64_t b = 0; b < nb; b++) {
             const int64_t n = hs64[b + 1] - hs64[b];
-            const int64_t k = std::max<int64_t>((n + len - 1) / len, 1);
-            if (k > 1) {
+            if (n <= len) continue;
+            const int64_t ng = (n + PT_WARPS * len - 1) / (PT_WARPS * len);
+            if (ng > 1) {
                 mb.push_back((int32_t) b);
                 mf.push_back(rows);
-                mn.push_back((int32_t) k);
+                mn.push_back((int32_t) ng);
             }
-            for (int64_t j = 0; j < k; j++) {
-                sb.push_back((int32_t) b);
-                lo.push_back((uint32_t) (hs64[b] + j * len));
-                hi.push_back((uint32_t) std::min<int64_t>(hs64[b] + (j + 1) * len, hs64[b + 1]));
-                so.push_back(k > 1 ? rows++ : -1);
-            }
+            const int64_t lb = ((n + ng * PT_WARPS - 1) / (ng * PT_WARPS) + 31) & ~(int64_t) 31;
+            for (int64_t j = 0; j < ng * PT_WARPS; j++)
+                slice(b, std::min(hs64[b] + j * lb, hs64[b + 1]), std::min(hs64[b] + (j + 1) * lb, hs64[b + 1]));
+            for (int64_t j = 0; j < ng; j++) go.push_back(ng > 1 ? rows++ : -1);
         }
+        // the other bins, PT_WARPS a group, each written by its warp
+        for (int64_t b = 0; b < nb; b++)
+            if (hs64[b + 1] - hs64[b] <= len) slice(b, hs64[b], hs64[b + 1]);
         B->nslices = (int64_t) sb.size();
+        go.resize((size_t) ((B->nslices + PT_WARPS - 1) / PT_WARPS), -2);
         B->nmulti = (int64_t) mb.size();
         B->slice_len = len;
         MDP_TRY(B->slice_bin.alloc(4 * sb.size()));
         MDP_TRY(B->slice_lo.alloc(4 * sb.size()));
         MDP_TRY(B->slice_hi.alloc(4 * sb.size()));
-        MDP_TRY(B->slice_out.alloc(4 * sb.size()));
+        MDP_TRY(B->group_out.alloc(4 * go.size()));
         MDP_CUDA(cudaMemcpy(B->slice_bin.p, sb.data(), 4 * sb.size(), cudaMemcpyHostToDevice));
         MDP_CUDA(cudaMemcpy(B->slice_lo.p, lo.data(), 4 * lo.size(), cudaMemcpyHostToDevice));
         MDP_CUDA(cudaMemcpy(B->slice_hi.p, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice));
-        MDP_CUDA(cudaMemcpy(B->slice_out.p, so.data(), 4 * so.size(), cudaMemcpyHostToDevice));
+        MDP_CUDA(cudaMemcpy(B->group_out.p, go.data(), 4 * go.size(), cudaMemcpyHostToDevice));
         if (!mb.empty()) {
             MDP_TRY(B->multi_bin.alloc(4 * mb.size()));
             MDP_TRY(B->multi_first.alloc(4 * mf.size()));
@@ -848,20 +865,25 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
 // x = P^T y over the slices of the bins' lists: warp k of a CTA owns slice
 // PT_WARPS*blockIdx.x + k.  TY/TW: TOD and weight types (double, or float for
 // the mixed solver's FP32 operator); products and sums in FP64.  U steps of 32
-// rows are loaded before they are added, for memory-level parallelism.  The
-// warp's sums go to the bin's map entries (a bin of one slice) or to the
-// slice's row of `partial`, summed by pt_partial_sum_kernel.
+// rows are loaded before they are added, for memory-level parallelism.  A CTA of
+// PT_WARPS bins of one slice writes their map entries; the warps of a CTA that all
+// work on one bin add up their sums in shared memory, in warp order, and write the
+// bin's entries or (a bin of several groups) the group's row of `partial`, summed by
+// pt_partial_sum_kernel.  Bound: DRAM, latency on short lists.  A partial map per slice
+// instead of one per group, and the row's offset gathered with its weights instead of the
+// pixel listed beside the row number, took 42.6 + 13.1 us for 4 x 2^20 rows and 49152 pixels.
 template <typename TY, typename TW>
 __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
-        const int32_t *__restrict__ off, const TW *__restrict__ w, const TY *__restrict__ y, double *__restrict__ x,
-        const uint32_t *__restrict__ perm, const int32_t *__restrict__ slice_bin, const uint32_t *__restrict__ slice_lo,
-        const uint32_t *__restrict__ slice_hi, const int32_t *__restrict__ slice_out, int64_t nslices,
+        const TW *__restrict__ w, const TY *__restrict__ y, double *__restrict__ x, const uint32_t *__restrict__ perm,
+        const uint8_t *__restrict__ pix, const int32_t *__restrict__ slice_bin, const uint32_t *__restrict__ slice_lo,
+        const uint32_t *__restrict__ slice_hi, const int32_t *__restrict__ group_out, int64_t nslices,
         double *__restrict__ partial, int64_t n_map) {
     constexpr int U = 4;
     __shared__ double acc_s[PT_WARPS][3 * PT_BIN_PIX];
     const int     wid = threadIdx.x >> 5, lane = lane_id();
     const int64_t sl = (int64_t) blockIdx.x * PT_WARPS + wid;
-    if (sl >= nslices) return;  // whole warps only; no CTA-wide barrier follows
+    const int     out = group_out[blockIdx.x];  // -2: a bin a warp; -1: one bin; else the row of `partial`
+    if (sl >= nslices) return;  // whole warps, only of the last group of kind -2: no barrier follows there
     double *acc = acc_s[wid];
     for (int i = lane; i < 3 * PT_BIN_PIX; i += 32) acc[i] = 0.0;
     __syncwarp();
@@ -871,30 +893,31 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
     // the row numbers of the next U steps are loaded while the current ones are
     // gathered and added: one memory latency per U steps on the warp's path
     uint32_t tn[U];
+    int      on[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const int64_t i = s0 + 32 * u + lane;
         tn[u] = (i < s1) ? perm[i] : 0u;
+        on[u] = (i < s1) ? 3 * (int) pix[i] : -1;
     }
     for (int64_t i0 = s0; i0 < s1; i0 += 32 * U) {
         uint32_t tc[U];
+        int      o[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             tc[u] = tn[u];
+            o[u] = on[u];
             const int64_t i = i0 + 32 * (U + u) + lane;
             tn[u] = (i < s1) ? perm[i] : 0u;
+            on[u] = (i < s1) ? 3 * (int) pix[i] : -1;
         }
-        int    o[U];
         double c0[U], c1[U], c2[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int64_t i = i0 + 32 * u + lane;
-            o[u] = -1;
             c0[u] = c1[u] = c2[u] = 0.0;
-            if (i < s1) {
+            if (o[u] >= 0) {
                 const int64_t t = tc[u];
                 const double  v = (double) y[t];
-                o[u] = (int) (off[t] - base);
                 c0[u] = (double) w[3 * t] * v;
                 c1[u] = (double) w[3 * t + 1] * v;
                 c2[u] = (double) w[3 * t + 2] * v;
@@ -948,17 +971,22 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
             __syncwarp();
         }
     }
-    const int out = slice_out[sl];
-    if (out < 0) {
-        const int64_t lim = min((int64_t) 3 * PT_BIN_PIX, n_map - base);
+    const int64_t lim = min((int64_t) 3 * PT_BIN_PIX, n_map - base);
+    if (out == -2) {
         for (int i = lane; i < lim; i += 32) x[base + i] = acc[i];
-    } else {
-        double *pr = partial + (int64_t) out * 3 * PT_BIN_PIX;
-        for (int i = lane; i < 3 * PT_BIN_PIX; i += 32) pr[i] = acc[i];
+        return;
+    }
+    __syncthreads();
+    double *dst = out < 0 ? x + base : partial + (int64_t) out * 3 * PT_BIN_PIX;
+    for (int i = threadIdx.x; i < (out < 0 ? (int) lim : 3 * PT_BIN_PIX); i += 32 * PT_WARPS) {
+        double v = acc_s[0][i];
+#pragma unroll
+        for (int k = 1; k < PT_WARPS; k++) v += acc_s[k][i];
+        dst[i] = v;
     }
 }
 
-// map entries of the bins of several slices: their partial maps summed in slice order
+// map entries of the bins of several groups: their partial maps summed in list order
 __global__ void pt_partial_sum_kernel(const double *__restrict__ partial, const int32_t *__restrict__ multi_bin,
                                       const int32_t *__restrict__ multi_first, const int32_t *__restrict__ multi_n,
                                       int64_t nmulti, double *__restrict__ x, int64_t n_map) {
@@ -982,8 +1010,8 @@ static int trmatvec_slices(mdp_context *ctx, const mdp_pointing *A, const TW *w,
     if (B.nslices > 0) {
         trmatvec_slices_kernel<TY, TW><<<(unsigned) ((B.nslices + PT_WARPS - 1) / PT_WARPS), 32 * PT_WARPS, 0,
                                          ctx->stream>>>(
-                A->off.as<int32_t>(), w, d_y, d_x, B.perm.as<uint32_t>(), B.slice_bin.as<int32_t>(),
-                B.slice_lo.as<uint32_t>(), B.slice_hi.as<uint32_t>(), B.slice_out.as<int32_t>(), B.nslices,
+                w, d_y, d_x, B.perm.as<uint32_t>(), B.pix.as<uint8_t>(), B.slice_bin.as<int32_t>(),
+                B.slice_lo.as<uint32_t>(), B.slice_hi.as<uint32_t>(), B.group_out.as<int32_t>(), B.nslices,
                 B.partial.as<double>(), A->n_map());
         MDP_CHECK_LAUNCH(ctx);
     }
