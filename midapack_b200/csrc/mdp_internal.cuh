@@ -117,11 +117,11 @@ struct mdp_pt_bins {
     DevBuf  start;   // int64 [nbins+1] offsets into perm
     DevBuf  perm;    // uint32 [valid rows] sample index, grouped by bin
     DevBuf  pix;     // uint8 [valid rows] the row's pixel inside its bin (with slices)
-    // slices of the bins' lists (P^T): every bin's list cut into runs of at
-    // most slice_len rows (one run for an empty bin), taken by the warps of groups (CTAs) of
+    // slices of the bins' lists (P^T): every bin's list in one run or cut into
+    // several, taken by the warps of groups (CTAs) of
     // eight: the slices of one long bin, of equal length, or eight bins of one slice.  A bin of several groups has partial maps, summed in order; they belong
     // to the pointing: two P^T of one pointing must not run at the same time.
-    int64_t nslices = 0, nmulti = 0, slice_len = 0;
+    int64_t nslices = 0, nmulti = 0;
     DevBuf  slice_bin;    // int32 [nslices]
     DevBuf  slice_lo;     // uint32 [nslices] first list entry
     DevBuf  slice_hi;     // uint32 [nslices] one past the last

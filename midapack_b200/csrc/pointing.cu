@@ -632,8 +632,8 @@ __global__ void trmatvec_general_kernel(const int32_t *__restrict__ local, const
 // the rows by bin, so the list is the same on every build): counts per
 // (row chunk, bin), bin totals, an exclusive scan over the bins, per-chunk
 // offsets within each bin, then one warp per row chunk writes its rows in
-// order.  Each bin's list is cut into slices of a fixed length (a function of
-// the row and bin counts only), and one warp owns one slice: it walks the
+// order.  Each bin's list is cut into slices (a function of the bins' row
+// counts only), and one warp owns one slice: it walks the
 // slice in order, 32 rows a step, and adds each row's three products into its
 // shared-memory copy of the bin's map.  A step whose offsets run strictly up
 // or down the lanes hits distinct pixels; in any other step the rows that hit
@@ -734,20 +734,45 @@ __global__ void __launch_bounds__(32) bin_chunk_scatter_kernel(const int32_t *__
     }
 }
 
-// rows per slice of the P^T bin lists: about 2^14 slices, enough to fill the
-// device whatever the map size, at least 512 and at most 2^16 rows each; a
-// function of the pointing alone (rows and bins), so that the sums are the
-// same on every device.  Longer slices would leave a small map's few bins to a few warps;
-// shorter ones write more partial maps (3 bin_pix doubles per PT_WARPS slices of a
-// bin cut in more).
-static int64_t pt_slice_len(int64_t m, int64_t nbins) {
-    int64_t len = 512;
-    while (len < (1 << 16) && m / len > (1 << 14)) len <<= 1;
-    // bins enough to fill the device by themselves: cut only the bins longer
-    // than the average (fewer partial maps to write and sum)
-    if (nbins >= 4096)
-        while (len < (1 << 16) && len < m / nbins) len <<= 1;
-    return len;
+// How the P^T bin lists are cut: the CTAs (groups of PT_WARPS warps) of each bin, 0 for a bin
+// that one warp takes.  A bin's CTAs are proportional to its rows, PT_WAVE k of them in all
+// (PT_WAVE: the CTAs resident at once), and bins of up to c/2 times a warp's rows go to one
+// warp, with (k, c) the cheapest of a few by whole waves times the longest warp's rows and a
+// constant for setting up and adding up its map (PT_FIXED rows' worth): a
+// wave begun for a few CTAs costs as much as a full one.  A function of the row counts alone,
+// so that the sums are the same on every device.  (Slices of a fixed power of two of rows
+// left 1.7 waves for 4 x 2^20 rows on 49152 pixels: 47 us.)
+#define PT_WAVE (4 * 148)
+#define PT_FIXED 192
+static std::vector<int32_t> pt_groups(const std::vector<int64_t> &start) {
+    const int64_t        nb = (int64_t) start.size() - 1, total = std::max<int64_t>(start[nb], 1);
+    std::vector<int32_t> best, g(nb);
+    double               best_cost = 0.0;
+    for (int kc : {103, 203, 303, 403, 603, 803, 1203, 1603, 108, 208, 408, 132, 232}) {
+        const int64_t k = kc / 100, c = kc % 100;
+        const int64_t warp_rows = std::max<int64_t>(total / (PT_WAVE * PT_WARPS * k), 128);
+        int64_t       ctas = 0, alone = 0, longest = 1;
+        for (int64_t b = 0; b < nb; b++) {
+            const int64_t n = start[b + 1] - start[b];
+            if (2 * n <= c * warp_rows) {
+                g[b] = 0;
+                alone++;
+                longest = std::max(longest, n);
+                continue;
+            }
+            const int64_t share = (n + warp_rows * PT_WARPS / 2) / (warp_rows * PT_WARPS);
+            g[b] = (int32_t) std::max<int64_t>(share, 1);
+            ctas += g[b];
+            longest = std::max(longest, n / ((int64_t) g[b] * PT_WARPS));
+        }
+        ctas += (alone + PT_WARPS - 1) / PT_WARPS;
+        const double cost = (double) ((ctas + PT_WAVE - 1) / PT_WAVE) * (double) (longest + PT_FIXED);
+        if (best.empty() || cost < best_cost) {
+            best = g;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *B, bool slices) {
@@ -806,7 +831,7 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
     MDP_CUDA(cudaMemcpy(B->start.p, hs64.data(), 8 * (nb + 1), cudaMemcpyHostToDevice));
     B->nslices = B->nmulti = 0;
     if (slices && nb > 0) {
-        const int64_t         len = pt_slice_len(A->m, nb);
+        const std::vector<int32_t> groups = pt_groups(hs64);
         std::vector<uint32_t> lo, hi;
         std::vector<int32_t>  sb, go, mb, mf, mn;
         int32_t               rows = 0;
@@ -818,9 +843,8 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
         // bins of several slices: groups of PT_WARPS slices, the bin's rows spread over them evenly
         // (whole steps of 32 rows), a group's output the bin itself or a partial map
         for (int64_t b = 0; b < nb; b++) {
-            const int64_t n = hs64[b + 1] - hs64[b];
-            if (n <= len) continue;
-            const int64_t ng = (n + PT_WARPS * len - 1) / (PT_WARPS * len);
+            const int64_t n = hs64[b + 1] - hs64[b], ng = groups[b];
+            if (ng == 0) continue;
             if (ng > 1) {
                 mb.push_back((int32_t) b);
                 mf.push_back(rows);
@@ -833,11 +857,10 @@ int mdp_build_bins(mdp_context *ctx, mdp_pointing *A, int bin_pix, mdp_pt_bins *
         }
         // the other bins, PT_WARPS a group, each written by its warp
         for (int64_t b = 0; b < nb; b++)
-            if (hs64[b + 1] - hs64[b] <= len) slice(b, hs64[b], hs64[b + 1]);
+            if (groups[b] == 0) slice(b, hs64[b], hs64[b + 1]);
         B->nslices = (int64_t) sb.size();
         go.resize((size_t) ((B->nslices + PT_WARPS - 1) / PT_WARPS), -2);
         B->nmulti = (int64_t) mb.size();
-        B->slice_len = len;
         MDP_TRY(B->slice_bin.alloc(4 * sb.size()));
         MDP_TRY(B->slice_lo.alloc(4 * sb.size()));
         MDP_TRY(B->slice_hi.alloc(4 * sb.size()));
