@@ -33,7 +33,7 @@
 
 #include "mdp_internal.cuh"
 
-#define MR_BLOCKS 296
+#define MR_BLOCKS 592
 #define MR_THREADS 256
 #define MR_MAXG 8
 #define MR_BIN_PIX 2048
@@ -248,29 +248,53 @@ __global__ void __launch_bounds__(512) mr_trmatvec32_kernel(const int32_t *__res
 }
 
 // ---------------------------------------------------------------- PCG kernels (interleaved)
+// The vectors of the batch are [npix][G][3]: item e = p G + j (pixel p, slot j) holds three
+// values at 3e.  One thread an item, so that a warp's loads are consecutive and a thread
+// keeps one slot (the grid's stride is a multiple of G).  With one thread a pixel, walking its
+// slots, 27840 pixels x 8 slots kept a third of the threads of one CTA an SM or two busy:
+// update 53 us, dot 18 us, direction 13 us.
+
 // h = gamma_j h + Cg_j for the slots that continue; H32 = FP32 copy of h for
 // every running slot
 template <int G>
-__global__ void mr_direction_kernel(double *__restrict__ H, float *__restrict__ H32, const double *__restrict__ CG,
-                                    int64_t npix, const int *__restrict__ run, const SlotScal *__restrict__ S) {
-    double gam[G];
-    bool   act[G], on[G];
+__global__ void __launch_bounds__(MR_THREADS) mr_direction_kernel(double *__restrict__ H, float *__restrict__ H32,
+                                                                 const double *__restrict__ CG, int64_t npix,
+                                                                 const int *__restrict__ run,
+                                                                 const SlotScal *__restrict__ S) {
+    const int j = threadIdx.x % G;
+    if (!run[j]) return;
+    const bool   act = S[j].cont != 0;
+    const double gam = S[j].gamma;
+    for (int64_t e = (int64_t) blockIdx.x * MR_THREADS + threadIdx.x; e < npix * G; e += (int64_t) gridDim.x * MR_THREADS) {
 #pragma unroll
-    for (int j = 0; j < G; j++) {
-        on[j] = run[j] != 0;
-        act[j] = on[j] && S[j].cont;
-        gam[j] = S[j].gamma;
-    }
-    const int64_t n = npix * 3 * G;
-    for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
-        const int j = (int) ((i / 3) % G);
-        if (!on[j]) continue;
-        double h = H[i];
-        if (act[j]) {
-            h = h * gam[j] + CG[i];
-            H[i] = h;
+        for (int k = 0; k < 3; k++) {
+            double h = H[3 * e + k];
+            if (act) {
+                h = h * gam + CG[3 * e + k];
+                H[3 * e + k] = h;
+            }
+            H32[3 * e + k] = (float) h;
         }
-        H32[i] = (float) h;
+    }
+}
+
+// K sums a thread, of the slot threadIdx.x % G: partials of slot j's sum k at part[k G + j]
+template <int G, int K>
+__device__ __forceinline__ void mr_slot_store(double (&v)[K], MRed *R) {
+    __shared__ double sh[K][G][MR_THREADS / 32];
+    const int         lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        for (int o = 16; o >= G; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane < G)
+#pragma unroll
+        for (int k = 0; k < K; k++) sh[k][lane][threadIdx.x >> 5] = v[k];
+    __syncthreads();
+    if (threadIdx.x < K * G) {
+        const int k = threadIdx.x / G, j = threadIdx.x % G;
+        double    s = 0.0;
+        for (int w = 0; w < MR_THREADS / 32; w++) s += sh[k][j][w];
+        R->part[threadIdx.x][blockIdx.x] = s;
     }
 }
 
@@ -283,15 +307,11 @@ __global__ void __launch_bounds__(MR_THREADS) mr_coeff_kernel(const double *__re
 #pragma unroll
     for (int j = 0; j < G; j++) any = any || run[j] != 0;
     if (!any) return;  // every slot has stopped: the whole grid returns
-    double v[G];
-#pragma unroll
-    for (int j = 0; j < G; j++) v[j] = 0.0;
-    for (int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (int64_t) gridDim.x * blockDim.x) {
-        const double *h = H + p * 3 * G, *q = Q + p * 3 * G;
-#pragma unroll
-        for (int j = 0; j < G; j++) v[j] += h[3 * j] * q[3 * j] + h[3 * j + 1] * q[3 * j + 1] + h[3 * j + 2] * q[3 * j + 2];
-    }
-    mr_block_store<G>(v, R);
+    double v[1] = {0.0};
+    if (run[threadIdx.x % G])
+        for (int64_t e = (int64_t) blockIdx.x * MR_THREADS + threadIdx.x; e < npix * G; e += (int64_t) gridDim.x * MR_THREADS)
+            v[0] += H[3 * e] * Q[3 * e] + H[3 * e + 1] * Q[3 * e + 1] + H[3 * e + 2] * Q[3 * e + 2];
+    mr_slot_store<G, 1>(v, R);
     if (mr_last_block(R, 0)) {
         const double *t = mr_sums<G>(R);
         if (threadIdx.x != 0) return;
@@ -313,47 +333,34 @@ __global__ void __launch_bounds__(MR_THREADS) mr_update_kernel(const double *__r
                                                               const double *__restrict__ GP, double *__restrict__ Gn,
                                                               double *__restrict__ CG, int64_t npix, int *run,
                                                               SlotScal *S, MRed *R) {
-    double ro[G];
-    bool   act[G], any = false;
+    bool any = false;
 #pragma unroll
-    for (int j = 0; j < G; j++) {
-        act[j] = run[j] != 0;
-        any = any || act[j];
-        ro[j] = S[j].ro;
-    }
+    for (int j = 0; j < G; j++) any = any || run[j] != 0;
     if (!any) return;  // every slot has stopped: the whole grid returns, no partials
-    double v[3 * G];
-#pragma unroll
-    for (int k = 0; k < 3 * G; k++) v[k] = 0.0;
-    for (int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (int64_t) gridDim.x * blockDim.x) {
-        const double *I = inv + 9 * p;
-        const double  i0 = I[0], i1 = I[1], i2 = I[2], i3 = I[3], i4 = I[4], i5 = I[5], i6 = I[6], i7 = I[7], i8 = I[8];
-#pragma unroll
-        for (int j = 0; j < G; j++) {
-            if (!act[j]) continue;
-            const int64_t e = (p * G + j) * 3;
-            double        gn[3], go[3];
+    const int    js = threadIdx.x % G;
+    const double ro = S[js].ro;
+    double       v[3] = {0.0, 0.0, 0.0};
+    if (run[js])
+        for (int64_t e = (int64_t) blockIdx.x * MR_THREADS + threadIdx.x; e < npix * G; e += (int64_t) gridDim.x * MR_THREADS) {
+            const double *I = inv + 9 * (e / G);
+            double        gn[3], go[3], c[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                DL[e + k] = DL[e + k] + ro[j] * H[e + k];
-                go[k] = GP[e + k];
-                gn[k] = go[k] - ro[j] * Q[e + k];
-                Gn[e + k] = gn[k];
+                DL[3 * e + k] = DL[3 * e + k] + ro * H[3 * e + k];
+                go[k] = GP[3 * e + k];
+                gn[k] = go[k] - ro * Q[3 * e + k];
+                Gn[3 * e + k] = gn[k];
             }
-            double c[3];
-            c[0] = i0 * gn[0] + i1 * gn[1] + i2 * gn[2];
-            c[1] = i3 * gn[0] + i4 * gn[1] + i5 * gn[2];
-            c[2] = i6 * gn[0] + i7 * gn[1] + i8 * gn[2];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                CG[e + k] = c[k];
-                v[j] += c[k] * gn[k];
-                v[G + j] += c[k] * (gn[k] - go[k]);
-                v[2 * G + j] += gn[k] * gn[k];
+                c[k] = I[3 * k] * gn[0] + I[3 * k + 1] * gn[1] + I[3 * k + 2] * gn[2];
+                CG[3 * e + k] = c[k];
+                v[0] += c[k] * gn[k];
+                v[1] += c[k] * (gn[k] - go[k]);
+                v[2] += gn[k] * gn[k];
             }
         }
-    }
-    mr_block_store<3 * G>(v, R);
+    mr_slot_store<G, 3>(v, R);
     if (mr_last_block(R, 1)) {
         const double *t = mr_sums<3 * G>(R);
         if (threadIdx.x != 0) return;
@@ -510,8 +517,8 @@ int launch_iteration(mdp_context *ctx, mdp_pointing *A, mdp_noise *N, Batch &B, 
     int         *run = B.run.as<int>();
     SlotScal    *S = B.scal.as<SlotScal>();
     MRed        *R = B.red.as<MRed>();
-    const int    gv = grid_for(B.npix * 3 * G, 256, ctx->sm_count * 8);
-    mr_direction_kernel<G><<<gv, 256, 0, st>>>(B.H.as<double>(), B.H32.as<float>(), B.CG.as<double>(), B.npix, run, S);
+    const int    gv = grid_for(B.npix * G, MR_THREADS, ctx->sm_count * 8);
+    mr_direction_kernel<G><<<gv, MR_THREADS, 0, st>>>(B.H.as<double>(), B.H32.as<float>(), B.CG.as<double>(), B.npix, run, S);
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(launch_apply32<G>(ctx, A, N, B, B.H32.as<float>()));
     mr_coeff_kernel<G><<<MR_BLOCKS, MR_THREADS, 0, st>>>(B.H.as<double>(), B.Q.as<double>(), B.npix, run, S, R);
