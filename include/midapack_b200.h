@@ -45,7 +45,10 @@ void     mdp_context_destroy(mdp_context *ctx);
 /* The solves keep their work buffers (TOD- and map-sized) in the context for
  * its next solve, so that repeated solves do not cudaMalloc/cudaFree (which
  * synchronise the device); mdp_context_trim frees them (after synchronising
- * the context's stream). */
+ * the context's stream).  Device memory that the library gives up (buffers of
+ * destroyed objects, temporaries) is kept for its next allocations, up to 2 GiB
+ * in blocks of up to 512 MiB for the process; mdp_context_trim gives that of the
+ * context's device back to the driver too. */
 int      mdp_context_trim(mdp_context *ctx);
 /* queue work on an existing cudaStream_t (e.g. the caller's; pass cudaStreamLegacy,
  * i.e. (void *) 1, for the legacy default stream); NULL = a stream of its own */

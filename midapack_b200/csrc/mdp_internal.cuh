@@ -6,6 +6,7 @@
 
 #include <cstdio>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "midapack_b200.h"
@@ -41,31 +42,36 @@ void mdp_set_error(const char *fmt, ...);
     } while (0)
 
 // ---------------------------------------------------------------- device buffer
+// Device memory by way of a process-wide cache of freed blocks (pointing.cu): setting an
+// operator up and closing it makes some seventy allocations, 0.1 ms each in the driver, and a
+// multi-RHS solve as many again.  A block enters the cache only after the device has finished
+// what was queued (as cudaFree waits), so any stream or thread may take it next.
+int  mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev);
+void mdp_mem_put(void *p, size_t bytes, int dev);
+void mdp_mem_trim(int dev);  // gives the device's cached blocks back to the driver
+
 struct DevBuf {
     void  *p     = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;  // of the block, at least what was asked for
+    int    dev   = 0;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p) mdp_mem_put(p, bytes, dev);
         p     = nullptr;
         bytes = 0;
     }
     int alloc(size_t nbytes) {  // (re)allocate when too small; contents are not kept
         if (nbytes <= bytes && p) return MDP_OK;
         release();
-        if (nbytes == 0) nbytes = 16;
-        cudaError_t e = cudaMalloc(&p, nbytes);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            cudaGetLastError();
-            mdp_set_error("cudaMalloc(%zu bytes): %s", nbytes, cudaGetErrorString(e));
-            return MDP_ENOMEM;
-        }
-        bytes = nbytes;
-        return MDP_OK;
+        return mdp_mem_get(nbytes == 0 ? 16 : nbytes, &p, &bytes, &dev);
+    }
+    void swap(DevBuf &o) {
+        std::swap(p, o.p);
+        std::swap(bytes, o.bytes);
+        std::swap(dev, o.dev);
     }
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
@@ -88,7 +94,7 @@ struct mdp_context {
     DevBuf       ws[13];    // [12]: FP32 (x, y, z, 0) copy of the map gathered by the FP32 P
     double      *h_pinned = nullptr;  // pinned host scalars
     // a second stream for launches that may overlap those on `stream`: forked from it and
-    // joined to it again within one call (mdp_side_fork / mdp_side_join), created on first use
+    // joined to it again within one call (mdp_side_fork / mdp_side_join)
     cudaStream_t side = nullptr;
     cudaEvent_t  side_ev[2] = {nullptr, nullptr};
     // optional per-operator timing inside the solver (CUDA events on the stream)

@@ -8,6 +8,8 @@
 // (sindex/dichotomy).
 #include <cstdarg>
 #include <cstring>
+#include <deque>
+#include <mutex>
 
 #include "mdp_internal.cuh"
 
@@ -37,6 +39,98 @@ extern "C" const char *mdp_strerror(int code) {
     }
 }
 
+// ============================================================== device memory
+// Freed blocks kept for the next allocation of about their size: blocks of up to
+// kMemBlock bytes, kMemCache bytes in all; beyond that the oldest go back to the
+// driver, all of a device's on mdp_context_trim or when the driver is out of memory.
+// Sizes are rounded up so that blocks fit again; a block is taken for a request of at
+// least three quarters of it.
+namespace {
+constexpr size_t kMemBlock = size_t(512) << 20, kMemCache = size_t(2) << 30;
+struct MemBlock {
+    void  *p;
+    size_t bytes;
+    int    dev;
+};
+std::mutex           g_mem_mu;
+std::deque<MemBlock> g_mem;  // oldest first
+size_t               g_mem_bytes = 0;
+
+size_t mem_round(size_t n) {
+    const size_t unit = n <= (1u << 16) ? 512 : n <= (1u << 20) ? (1u << 14) : (1u << 20);
+    return (n + unit - 1) / unit * unit;
+}
+// drops the oldest blocks (of device dev, or of all: dev < 0) until at most `keep` bytes are cached
+void mem_drop(int dev, size_t keep) {
+    for (auto it = g_mem.begin(); it != g_mem.end() && g_mem_bytes > keep;) {
+        if (dev >= 0 && it->dev != dev) {
+            ++it;
+            continue;
+        }
+        g_mem_bytes -= it->bytes;
+        cudaFree(it->p);
+        it = g_mem.erase(it);
+    }
+}
+}  // namespace
+
+int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
+    const size_t want = mem_round(nbytes);
+    *p = nullptr;
+    *got = 0;
+    MDP_CUDA(cudaGetDevice(dev));
+    std::lock_guard<std::mutex> lk(g_mem_mu);
+    auto best = g_mem.end();
+    for (auto it = g_mem.begin(); it != g_mem.end(); ++it)
+        if (it->dev == *dev && it->bytes >= want && want >= it->bytes / 4 * 3 && (best == g_mem.end() || it->bytes < best->bytes))
+            best = it;
+    if (best != g_mem.end()) {
+        *p = best->p;
+        *got = best->bytes;
+        g_mem_bytes -= best->bytes;
+        g_mem.erase(best);
+        return MDP_OK;
+    }
+    cudaError_t e = cudaMalloc(p, want);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        mem_drop(*dev, 0);
+        e = cudaMalloc(p, want);
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+        mdp_set_error("cudaMalloc(%zu bytes): %s", nbytes, cudaGetErrorString(e));
+        return MDP_ENOMEM;
+    }
+    *got = want;
+    return MDP_OK;
+}
+
+void mdp_mem_put(void *p, size_t bytes, int dev) {
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    // what was queued on the block is over before anyone can take it again
+    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lk(g_mem_mu);
+        if (!ok || bytes > kMemBlock) {
+            cudaFree(p);
+        } else {
+            g_mem.push_back(MemBlock{p, bytes, dev});
+            g_mem_bytes += bytes;
+            mem_drop(-1, kMemCache);
+        }
+    }
+    if (cur != dev) cudaSetDevice(cur);
+}
+
+void mdp_mem_trim(int dev) {
+    std::lock_guard<std::mutex> lk(g_mem_mu);
+    mem_drop(dev, 0);
+}
+
 // ============================================================== context
 extern "C" int mdp_context_create(int device, mdp_context **out) {
     if (!out) return MDP_EINVAL;
@@ -64,6 +158,14 @@ extern "C" int mdp_context_create(int device, mdp_context **out) {
         mdp_set_error("cudaMallocHost failed");
         return MDP_ENOMEM;
     }
+    // the side stream here and not on first use, which may be inside a graph capture
+    if (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->side_ev[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->side_ev[1], cudaEventDisableTiming) != cudaSuccess) {
+        mdp_context_destroy(ctx);
+        mdp_set_error("cudaStreamCreate failed");
+        return MDP_ECUDA;
+    }
     *out = ctx;
     return MDP_OK;
 }
@@ -75,6 +177,7 @@ extern "C" int mdp_context_trim(mdp_context *ctx) {
     for (DevBuf &b : ctx->ws) b.release();
     ctx->scratch.release();
     ctx->scratch2.release();
+    mdp_mem_trim(ctx->device);
     return MDP_OK;
 }
 
@@ -107,10 +210,6 @@ extern "C" int mdp_context_set_stream(mdp_context *ctx, void *cuda_stream) {
 }
 
 int mdp_side_fork(mdp_context *ctx) {
-    if (!ctx->side) {
-        for (cudaEvent_t &e : ctx->side_ev) MDP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        MDP_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-    }
     MDP_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
     MDP_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
     return MDP_OK;

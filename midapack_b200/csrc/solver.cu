@@ -760,10 +760,10 @@ int mdp_bj_build(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, BJState 
     MDP_CUDA(cudaStreamSynchronize(st));
     bj->ncut = h_ncut;
     if (h_ncut == 0) {
-        std::swap(bj->inv.p, inv.p), std::swap(bj->inv.bytes, inv.bytes);
-        std::swap(bj->W.p, W.p), std::swap(bj->W.bytes, W.bytes);
-        std::swap(bj->rcond.p, rcond.p), std::swap(bj->rcond.bytes, rcond.bytes);
-        std::swap(bj->hits.p, hits.p), std::swap(bj->hits.bytes, hits.bytes);
+        bj->inv.swap(inv);
+        bj->W.swap(W);
+        bj->rcond.swap(rcond);
+        bj->hits.swap(hits);
         bj->npix = npix0;
         return MDP_OK;
     }
@@ -805,8 +805,7 @@ int mdp_bj_build(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, BJState 
                                               bj->rcond.as<double>(), bj->hits.as<int32_t>());
     MDP_CHECK_LAUNCH(ctx);
     MDP_CUDA(cudaStreamSynchronize(st));
-    std::swap(A->lindices.p, lind2.p);
-    std::swap(A->lindices.bytes, lind2.bytes);
+    A->lindices.swap(lind2);
     A->bins.valid = 0;  // pixels were renumbered
     A->mbins.valid = 0;
     A->trash_pix = 1;
@@ -1269,8 +1268,7 @@ extern "C" int mdp_pointing_cut(mdp_context *ctx, mdp_pointing *A, const int32_t
                                             remap.as<uint32_t>(), lind2.as<int32_t>());
     MDP_CHECK_LAUNCH(ctx);
     MDP_CUDA(cudaStreamSynchronize(st));
-    std::swap(A->lindices.p, lind2.p);
-    std::swap(A->lindices.bytes, lind2.bytes);
+    A->lindices.swap(lind2);
     A->bins.valid = 0;
     A->mbins.valid = 0;
     A->trash_pix = 1;
