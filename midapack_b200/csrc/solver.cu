@@ -735,6 +735,16 @@ __global__ void pcg_direction_kernel(double *__restrict__ h, const double *__res
         h[i] = h[i] * gamma + Cg[i];
 }
 
+// rows past the last noise block: N^-1 leaves them as they are (mdp_stbmm writes the rows up
+// to the end of the blocks only)
+template <typename T>
+static int pass_tail(mdp_context *ctx, const mdp_noise *N, int64_t m, const T *in, T *out) {
+    if (N->nrow_end < m)
+        MDP_CUDA(cudaMemcpyAsync(out + N->nrow_end, in + N->nrow_end, sizeof(T) * (m - N->nrow_end),
+                                 cudaMemcpyDeviceToDevice, ctx->stream));
+    return MDP_OK;
+}
+
 // ================================================================= the solve
 int mdp_bj_build(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, BJState *bj) {
     if (!A->triplet) {
@@ -847,6 +857,7 @@ int mdp_pcg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
         MDP_TRY(mdp_templates_filter(ctx, tpl, ta, tb));
     else
         MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, nullptr));
+    if (!tpl) MDP_TRY(pass_tail(ctx, N, m, ta, tb));
     MDP_TRY(mdp_trmatvec_launch(ctx, A, tb, g));
     if (tl) {
         MDP_TRY(mdp_twolevel_qtx(ctx, tl, g));
@@ -886,6 +897,7 @@ int mdp_pcg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
             MDP_TRY(mdp_templates_filter(ctx, tpl, ta, tb));
         else
             MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, fused == MDP_OK ? N->means.as<double>() : nullptr));
+        if (!tpl) MDP_TRY(pass_tail(ctx, N, m, ta, tb));
         if (prof) cudaEventRecord(ctx->ev[2], st);
         MDP_TRY(mdp_trmatvec_launch(ctx, A, tb, q));
         if (prof) cudaEventRecord(ctx->ev[3], st);
@@ -1079,6 +1091,7 @@ extern "C" int mdp_gls_solve_mixed(mdp_context *ctx, mdp_pointing *A, const mdp_
         tod_residual_kernel<<<gm, 256, 0, st>>>(A->off.as<int32_t>(), d_signal, d_noise, ta, m);
         MDP_CHECK_LAUNCH(ctx);
         MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, nullptr));
+        MDP_TRY(pass_tail(ctx, N, m, ta, tb));
         MDP_TRY(mdp_trmatvec_launch(ctx, A, tb, r));
         dot_self_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(r, n, S);
         MDP_CHECK_LAUNCH(ctx);
@@ -1131,6 +1144,7 @@ extern "C" int mdp_gls_solve_mixed(mdp_context *ctx, mdp_pointing *A, const mdp_
             if (fused == MDP_EUNSUPPORTED) MDP_TRY(mdp_matvec32_launch(ctx, A, h, fa));
             if (prof) cudaEventRecord(ctx->ev[1], st);
             MDP_TRY(mdp_stbmm_impl32(ctx, N, fa, fb, fused == MDP_OK ? N->means.as<double>() : nullptr));
+            MDP_TRY(pass_tail(ctx, N, m, fa, fb));
             if (prof) cudaEventRecord(ctx->ev[2], st);
             MDP_TRY(mdp_trmatvec32_launch(ctx, A, fb, q));
             if (prof) cudaEventRecord(ctx->ev[3], st);
@@ -1289,6 +1303,7 @@ int mdp_gls_rhs(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
                                                                                d_noise, ta, m);
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, nullptr));
+    MDP_TRY(pass_tail(ctx, N, m, ta, tb));
     return mdp_trmatvec_launch(ctx, A, tb, d_g);
 }
 
@@ -1302,6 +1317,7 @@ int mdp_apply_op_impl(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, con
     if (fused != MDP_OK && fused != MDP_EUNSUPPORTED) return fused;
     if (fused == MDP_EUNSUPPORTED) MDP_TRY(mdp_matvec_launch(ctx, A, d_h, ta));
     MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, fused == MDP_OK ? N->means.as<double>() : nullptr));
+    MDP_TRY(pass_tail(ctx, N, m, ta, tb));
     return mdp_trmatvec_launch(ctx, A, tb, d_q);
 }
 
@@ -1324,6 +1340,7 @@ extern "C" int mdp_gls_residual(mdp_context *ctx, mdp_pointing *A, const mdp_noi
     tod_residual_kernel<<<gm, 256, 0, st>>>(A->off.as<int32_t>(), d_signal, d_noise, ta, m);
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(mdp_stbmm_impl(ctx, N, ta, tb, nullptr));
+    MDP_TRY(pass_tail(ctx, N, m, ta, tb));
     return mdp_trmatvec_launch(ctx, A, tb, d_r);
 }
 
@@ -1347,5 +1364,6 @@ extern "C" int mdp_apply_op(mdp_context *ctx, mdp_pointing *A, const mdp_noise *
     if (fused != MDP_OK && fused != MDP_EUNSUPPORTED) return fused;
     if (fused == MDP_EUNSUPPORTED) MDP_TRY(mdp_matvec32_launch(ctx, A, d_h, fa));
     MDP_TRY(mdp_stbmm_impl32(ctx, N, fa, fb, fused == MDP_OK ? N->means.as<double>() : nullptr));
+    MDP_TRY(pass_tail(ctx, N, m, fa, fb));
     return mdp_trmatvec32_launch(ctx, A, fb, d_q);
 }

@@ -11,13 +11,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("sizes", [[1], [2, 1, 3, 1], [2047, 2049, 1, 4098, 2], [4096, 2048, 6145]])
-def test_operator_over_chunk_edges(gpu_ctx, sizes, shift):
+@pytest.mark.parametrize("sizes,tail", [([1], 0), ([2, 1, 3, 1], 0), ([2047, 2049, 1, 4098, 2], 0), ([4096, 2048, 6145], 0),
+                                        ([500, 700], 333)])   # rows past the last block pass through N^-1
+def test_operator_over_chunk_edges(gpu_ctx, sizes, tail, shift):
     import torch
     import midapack_b200 as mb
     from midapack_b200.dist import GpuShard
     rng = np.random.default_rng(len(sizes) + shift)
-    m, npix, lam = int(sum(sizes)), 40, 2
+    m, npix, lam = int(sum(sizes)) + tail, 40, 2
     p = rng.integers(0, npix, m)
     p[rng.random(m) < 0.05] = -1
     p[0] = 3

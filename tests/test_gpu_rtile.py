@@ -34,7 +34,7 @@ def _row(rng, lam):
     (2048, [20000, 4100, 65537], "r,1,12"),
     (5000, [40000, 9001], "r,2,12"),
     (8192, [70000, 8191], "r,3,12"),
-    (16384, [140000, 3 * 16384 + 1], "r,4,12"),
+    (16384, [70001, 16383], "r,4,12"),
     (2, [300001], "r,4,12"),                  # windows that end past the block by most of a tile
 ])
 def test_right_angle_tiles_vs_exact(gpu_ctx, lam, sizes, plan):
