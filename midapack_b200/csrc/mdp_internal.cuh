@@ -194,6 +194,56 @@ struct mdp_tile_plan {
     }
 };
 
+// The row chunks of the block means, for the kernels that sum them (one CTA a chunk)
+struct mdp_chunks {
+    const int64_t *start;                 // [n_chunks]
+    const int32_t *len, *blk;             // [n_chunks]
+    const int32_t *blk_chunk0, *blk_nchunk, *blk_len;  // [nb]
+    uint32_t      *arrived;               // [nb]
+    double        *partial, *means;
+};
+
+// The end of a CTA that has summed its chunk blockIdx.x: its partial sum from the threads' acc,
+// and the block's mean by the CTA that finishes the block's last chunk (the partial sums in a
+// fixed order: lane l takes l, l + 32, ..., then the lanes pairwise).  All threads of the CTA, at
+// most 1024.  `arrived` counts modulo the block's chunks, so that it needs no reset; null: the
+// partial sum only, the means are a kernel of their own.  That is the rule above MDP_MEAN_CHUNKS
+// chunks (one wave of CTAs): the fence and the count keep a CTA's slot for 1-2 us, which a
+// second wave waits for (P of 8 x 2^20 rows: 5 us more than the 4 us of the other kernel);
+// within one wave nothing waits (four blocks of 12000 rows, N^-1 in all 16.4 -> 14.3 us).
+#define MDP_MEAN_CHUNKS (4 * 148)
+__device__ __forceinline__ void chunk_mean(const mdp_chunks &c, double acc) {
+    __shared__ double ws[32];
+    const int         lane = threadIdx.x & 31;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) ws[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    double v = lane < (int) (blockDim.x >> 5) ? ws[lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (!c.arrived) {
+        if (lane == 0) c.partial[blockIdx.x] = v;
+        return;
+    }
+    const int b = c.blk[blockIdx.x], n = c.blk_nchunk[b];
+    if (n > 1) {
+        uint32_t prev = 0;
+        if (lane == 0) {
+            c.partial[blockIdx.x] = v;
+            __threadfence();
+            prev = atomicAdd(c.arrived + b, 1u);
+        }
+        prev = __shfl_sync(0xffffffffu, prev, 0);
+        if ((prev + 1u) % (uint32_t) n != 0u) return;
+        __threadfence();
+        const double *p = c.partial + c.blk_chunk0[b];
+        v = 0.0;
+        for (int i = lane; i < n; i += 32) v += __ldcg(p + i);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    if (lane == 0) c.means[b] = v / (double) c.blk_len[b];
+}
+
 // window of a right-angle tile (rtile.cu)
 struct alignas(16) mdp_rtile {
     int64_t start;             // first row of the tile's block
@@ -227,7 +277,15 @@ struct mdp_noise {
     DevBuf               chunk_len;      // int32 [n_chunks]
     DevBuf               blk_chunk0;     // int32 [nb] first chunk of each block
     DevBuf               blk_nchunk;     // int32 [nb]
+    DevBuf               chunk_blk;      // int32 [n_chunks] block of each chunk
+    DevBuf               arrived;        // uint32 [nb] chunks of a block finished, modulo its chunks
     DevBuf               partial;        // double [n_chunks] chunk sums
+    mdp_chunks           chunks(double *d_partial, double *d_means) const {
+        return mdp_chunks{chunk_start.as<int64_t>(), chunk_len.as<int32_t>(), chunk_blk.as<int32_t>(),
+                          blk_chunk0.as<int32_t>(), blk_nchunk.as<int32_t>(), blk_len.as<int32_t>(),
+                          n_chunks <= MDP_MEAN_CHUNKS ? arrived.as<uint32_t>() : nullptr, d_partial, d_means};
+    }
+    mdp_chunks           chunks() const { return chunks(partial.as<double>(), means.as<double>()); }
 };
 
 // ---------------------------------------------------------------- two-level preconditioner (twolevel.cu)
@@ -274,6 +332,8 @@ int mdp_exclusive_scan_u32(mdp_context *ctx, const uint32_t *d_in, uint32_t *d_o
                            uint32_t *h_total);
 int mdp_stbmm_impl(mdp_context *ctx, const mdp_noise *N, const double *d_in, double *d_out,
                    const double *d_means_or_null);
+// the block means of ncols columns ([ncols][n_chunks] chunk sums) unless the chunks' kernel takes them
+int mdp_means_final(mdp_context *ctx, const mdp_noise *N, const mdp_chunks &c, int ncols);
 int mdp_block_means(mdp_context *ctx, const mdp_noise *N, const double *d_v, double *d_means);
 // spectrum of the reference's circulant embedding of T (circ_init_fftw), bs/2+1 complex into h_F
 int mdp_circulant_spectrum(mdp_context *ctx, const double *h_T, int lambda, int bs, double *h_F);
@@ -310,8 +370,6 @@ int mdp_noise_prepare_fp32(mdp_context *ctx, mdp_noise *N);
 int mdp_stbmm_impl32(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d_out, const double *d_means);
 int mdp_stbmm32_batch(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d_out, int ncols,
                       int64_t col_stride, const double *d_means, const int *d_active);
-int mdp_noise_chunks(const mdp_noise *N, int *n_chunks, const int64_t **d_chunk_start, const int32_t **d_chunk_len,
-                     const int32_t **d_blk_chunk0, const int32_t **d_blk_nchunk, int *covers_all);
 int mdp_pointing_prepare_fp32(mdp_context *ctx, mdp_pointing *A);
 int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noise *N, const double *d_x,
                             float *d_y);

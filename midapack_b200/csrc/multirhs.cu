@@ -99,10 +99,8 @@ __device__ __forceinline__ const double *mr_sums(const MRed *R) {
 template <int G>
 __global__ void __launch_bounds__(512) mr_matvec32_kernel(const int32_t *__restrict__ off, const float *__restrict__ w,
                                                           const float *__restrict__ H, const int *__restrict__ run,
-                                                          float *__restrict__ Y, int64_t m,
-                                                          const int64_t *__restrict__ chunk_start,
-                                                          const int32_t *__restrict__ chunk_len, int n_chunks,
-                                                          double *__restrict__ partial) {
+                                                          float *__restrict__ Y, int64_t m, mdp_chunks c,
+                                                          int n_chunks, int nb) {
     bool act[G], any = false;
 #pragma unroll
     for (int j = 0; j < G; j++) {
@@ -110,8 +108,8 @@ __global__ void __launch_bounds__(512) mr_matvec32_kernel(const int32_t *__restr
         any = any || act[j];
     }
     if (!any) return;  // every slot has stopped
-    const int64_t s = chunk_start[blockIdx.x];
-    const int     n = chunk_len[blockIdx.x];
+    const int64_t s = c.start[blockIdx.x];
+    const int     n = c.len[blockIdx.x];
     double        acc[G];
 #pragma unroll
     for (int j = 0; j < G; j++) acc[j] = 0.0;
@@ -168,22 +166,28 @@ __global__ void __launch_bounds__(512) mr_matvec32_kernel(const int32_t *__restr
     if (threadIdx.x < G) {
         double v = 0.0;
         for (int q = 0; q < (int) (blockDim.x >> 5); q++) v += ws[threadIdx.x][q];
-        partial[(int64_t) threadIdx.x * n_chunks + blockIdx.x] = v;
+        c.partial[(int64_t) threadIdx.x * n_chunks + blockIdx.x] = v;
     }
-}
-
-// block means of every slot from its chunk sums, a warp a block
-__global__ void mr_means_kernel(const double *__restrict__ partial, int n_chunks, const int32_t *__restrict__ blk_chunk0,
-                                const int32_t *__restrict__ blk_nchunk, const int32_t *__restrict__ blk_len, int nb,
-                                double *__restrict__ means) {
-    const int j = blockIdx.y, lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
-    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nw) {
-        const int     n = blk_nchunk[b];
-        const double *p = partial + (int64_t) j * n_chunks + blk_chunk0[b];
-        double        s = 0.0;
-        for (int c = lane; c < n; c += 32) s += p[c];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) means[(int64_t) j * nb + b] = s / (double) blk_len[b];
+    // the CTA that finishes the block's last chunk takes the block's mean of every slot (as
+    // chunk_mean does for one)
+    if (!c.arrived) return;
+    __shared__ bool is_last;
+    const int       b = c.blk[blockIdx.x], nc = c.blk_nchunk[b];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = (atomicAdd(c.arrived + b, 1u) + 1u) % (uint32_t) nc == 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!is_last) return;
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < G; j += (int) (blockDim.x >> 5)) {
+        const double *p = c.partial + (int64_t) j * n_chunks + c.blk_chunk0[b];
+        double        v = 0.0;
+        for (int i = lane; i < nc; i += 32) v += __ldcg(p + i);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) c.means[(int64_t) j * nb + b] = v / (double) c.blk_len[b];
     }
 }
 
@@ -479,8 +483,6 @@ struct Batch {
     DevBuf  run;                   // int [G]
     DevBuf  scal, red;             // SlotScal [G], MRed
     int     n_chunks = 0;
-    const int64_t *chunk_start = nullptr;
-    const int32_t *chunk_len = nullptr, *blk_chunk0 = nullptr, *blk_nchunk = nullptr;
 };
 
 template <int G>
@@ -488,14 +490,10 @@ int launch_apply32(mdp_context *ctx, mdp_pointing *A, mdp_noise *N, Batch &B, co
     cudaStream_t st = ctx->stream;
     const int   *run = B.run.as<int>();
     mr_matvec32_kernel<G><<<B.n_chunks, 512, 0, st>>>(A->off.as<int32_t>(), A->w32.as<float>(), h, run, B.Y.as<float>(),
-                                                      B.m, B.chunk_start, B.chunk_len, B.n_chunks,
-                                                      B.partial.as<double>());
+                                                      B.m, N->chunks(B.partial.as<double>(), B.means.as<double>()),
+                                                      B.n_chunks, N->nb);
     MDP_CHECK_LAUNCH(ctx);
-    mr_means_kernel<<<dim3(grid_for(N->nb, 4, 256), G), 128, 0, st>>>(B.partial.as<double>(), B.n_chunks,
-                                                                       B.blk_chunk0, B.blk_nchunk,
-                                                                       N->blk_len.as<int32_t>(), N->nb,
-                                                                       B.means.as<double>());
-    MDP_CHECK_LAUNCH(ctx);
+    MDP_TRY(mdp_means_final(ctx, N, N->chunks(B.partial.as<double>(), B.means.as<double>()), G));
     MDP_TRY(mdp_stbmm32_batch(ctx, N, B.Y.as<float>(), B.Z.as<float>(), G, B.m, B.means.as<double>(), run));
     MDP_CUDA(cudaMemsetAsync(B.Q.p, 0, sizeof(double) * B.npix * 3 * G, st));
     if (A->mbins.nbins > 0) {
@@ -546,8 +544,7 @@ int alloc_batch(mdp_context *ctx, mdp_pointing *A, mdp_noise *N, int G, int64_t 
     B.m = A->m;
     B.npix = npix;
     B.nmap = 3 * npix;
-    int covers = 0;
-    MDP_TRY(mdp_noise_chunks(N, &B.n_chunks, &B.chunk_start, &B.chunk_len, &B.blk_chunk0, &B.blk_nchunk, &covers));
+    B.n_chunks = N->n_chunks;
     const size_t nv = sizeof(double) * (size_t) std::max<int64_t>(npix, 1) * 3 * G;
     for (DevBuf *b : {&B.H, &B.Q, &B.G1, &B.G2, &B.CG, &B.DL}) MDP_TRY(b->alloc(nv));
     for (DevBuf *b : {&B.H, &B.Q, &B.G1, &B.G2, &B.CG, &B.DL}) MDP_CUDA(cudaMemsetAsync(b->p, 0, nv, ctx->stream));
@@ -821,15 +818,9 @@ extern "C" int mdp_gls_solve_multi(mdp_context *ctx, mdp_pointing *A, const mdp_
         mdp_set_error("mdp_gls_solve_multi: the noise blocks must cover every pointing row and lambda > 1");
         return MDP_EUNSUPPORTED;
     }
-    {
-        int            nc = 0, covers = 0;
-        const int64_t *a;
-        const int32_t *b, *c, *d;
-        MDP_TRY(mdp_noise_chunks(N, &nc, &a, &b, &c, &d, &covers));
-        if (!covers) {
-            mdp_set_error("mdp_gls_solve_multi: the noise blocks must cover every pointing row");
-            return MDP_EUNSUPPORTED;
-        }
+    if (!N->covers_all) {
+        mdp_set_error("mdp_gls_solve_multi: the noise blocks must cover every pointing row");
+        return MDP_EUNSUPPORTED;
     }
     MDP_CUDA(cudaSetDevice(ctx->device));
     auto    tp0 = std::chrono::steady_clock::now();

@@ -1035,41 +1035,31 @@ static size_t tile_smem(int log_ml) {
 
 // ------------------------------------------------------------------ block means and white noise
 template <typename T>
-__global__ void block_partial_sums(const T *__restrict__ v, const int64_t *__restrict__ chunk_start,
-                                   const int32_t *__restrict__ chunk_len, double *__restrict__ partial) {
-    const int64_t s = chunk_start[blockIdx.x];
-    const int     n = chunk_len[blockIdx.x];
+__global__ void __launch_bounds__(512) block_means_kernel(const T *__restrict__ v, mdp_chunks c) {
+    const int64_t s = c.start[blockIdx.x];
+    const int     n = c.len[blockIdx.x];
     double        acc = 0.0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) acc += (double) v[s + j];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double x = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = x;
-    }
+    chunk_mean(c, acc);
 }
 
-// the mean of every block from its chunk sums, a warp a block (lane l adds chunks l, l + 32, ...,
-// then the lanes pairwise)
-__global__ void block_means_final(const double *__restrict__ partial, const int32_t *__restrict__ blk_chunk0,
-                                  const int32_t *__restrict__ blk_nchunk, const int32_t *__restrict__ blk_len,
-                                  int nb, double *__restrict__ means) {
+// the mean of every block from its chunk sums, a warp a block, column blockIdx.y of a batch
+__global__ void block_means_final(mdp_chunks c, int n_chunks, int nb) {
     const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
     for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nw) {
-        const int     n = blk_nchunk[b];
-        const double *p = partial + blk_chunk0[b];
+        const int     n = c.blk_nchunk[b];
+        const double *p = c.partial + (int64_t) blockIdx.y * n_chunks + c.blk_chunk0[b];
         double        s = 0.0;
-        for (int c = lane; c < n; c += 32) s += p[c];
+        for (int i = lane; i < n; i += 32) s += p[i];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) means[b] = s / (double) blk_len[b];
+        if (lane == 0) c.means[(int64_t) blockIdx.y * nb + b] = s / (double) c.blk_len[b];
     }
 }
-static void launch_means_final(mdp_context *ctx, const mdp_noise *N, const double *partial, double *means) {
-    block_means_final<<<grid_for(N->nb, 4, 2048), 128, 0, ctx->stream>>>(
-            partial, N->blk_chunk0.as<int32_t>(), N->blk_nchunk.as<int32_t>(), N->blk_len.as<int32_t>(), N->nb, means);
+int mdp_means_final(mdp_context *ctx, const mdp_noise *N, const mdp_chunks &c, int ncols) {
+    if (c.arrived) return MDP_OK;  // taken by the chunks' kernel
+    block_means_final<<<dim3(grid_for(N->nb, 4, 2048), ncols), 128, 0, ctx->stream>>>(c, N->n_chunks, N->nb);
+    MDP_CHECK_LAUNCH(ctx);
+    return MDP_OK;
 }
 
 __global__ void white_kernel(const double *__restrict__ vin, double *__restrict__ vout, const int64_t *__restrict__ bstart,
@@ -1773,11 +1763,12 @@ extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *
         if (n_ch >= 8 * ctx->sm_count) break;
     }
     std::vector<int64_t> cs;
-    std::vector<int32_t> cl, c0(nb_blocks), cn(nb_blocks);
+    std::vector<int32_t> cl, cb, c0(nb_blocks), cn(nb_blocks);
     for (int b = 0; b < nb_blocks; b++) {
         c0[b] = (int32_t) cs.size();
         for (int64_t o = 0; o < h_n[b]; o += CH) {
             cs.push_back(h_idv[b] + o);
+            cb.push_back(b);
             cl.push_back((int32_t) std::min<int64_t>(CH, h_n[b] - o));
         }
         cn[b] = (int32_t) cs.size() - c0[b];
@@ -1785,11 +1776,14 @@ extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *
     N->n_chunks = (int) cs.size();
     if ((rc = N->chunk_start.alloc(8 * std::max<size_t>(cs.size(), 1))) ||
         (rc = N->chunk_len.alloc(4 * std::max<size_t>(cl.size(), 1))) || (rc = N->blk_chunk0.alloc(4 * nb_blocks)) ||
-        (rc = N->blk_nchunk.alloc(4 * nb_blocks)) || (rc = N->partial.alloc(8 * std::max<size_t>(cs.size(), 1))))
+        (rc = N->blk_nchunk.alloc(4 * nb_blocks)) || (rc = N->partial.alloc(8 * std::max<size_t>(cs.size(), 1))) ||
+        (rc = N->chunk_blk.alloc(4 * std::max<size_t>(cb.size(), 1))) || (rc = N->arrived.alloc(4 * nb_blocks)))
         return fail(rc);
+    cudaMemset(N->arrived.p, 0, 4 * nb_blocks);
     if (!cs.empty()) {
         cudaMemcpy(N->chunk_start.p, cs.data(), 8 * cs.size(), cudaMemcpyHostToDevice);
         cudaMemcpy(N->chunk_len.p, cl.data(), 4 * cl.size(), cudaMemcpyHostToDevice);
+        cudaMemcpy(N->chunk_blk.p, cb.data(), 4 * cb.size(), cudaMemcpyHostToDevice);
     }
     cudaMemcpy(N->blk_chunk0.p, c0.data(), 4 * nb_blocks, cudaMemcpyHostToDevice);
     cudaMemcpy(N->blk_nchunk.p, cn.data(), 4 * nb_blocks, cudaMemcpyHostToDevice);
@@ -1848,11 +1842,10 @@ int mdp_block_means(mdp_context *ctx, const mdp_noise *N, const double *d_v, dou
         MDP_CUDA(cudaMemsetAsync(d_means, 0, 8 * N->nb, ctx->stream));
         return MDP_OK;
     }
-    block_partial_sums<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_v, N->chunk_start.as<int64_t>(),
-                                                             N->chunk_len.as<int32_t>(), N->partial.as<double>());
+    const mdp_chunks c = N->chunks(N->partial.as<double>(), d_means);
+    block_means_kernel<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_v, c);
     MDP_CHECK_LAUNCH(ctx);
-    launch_means_final(ctx, N, N->partial.as<double>(), d_means);
-    MDP_CHECK_LAUNCH(ctx);
+    MDP_TRY(mdp_means_final(ctx, N, c, 1));
     return MDP_OK;
 }
 
@@ -1886,11 +1879,9 @@ template <bool VEC>
 __global__ void __launch_bounds__(512) matvec_chunk_sums_kernel(const int32_t *__restrict__ off,
                                                                 const double *__restrict__ w,
                                                                 const double *__restrict__ x, double *__restrict__ y,
-                                                                const int64_t *__restrict__ chunk_start,
-                                                                const int32_t *__restrict__ chunk_len,
-                                                                double *__restrict__ partial) {
-    const int64_t s = chunk_start[blockIdx.x];
-    const int64_t e = s + chunk_len[blockIdx.x];
+                                                                mdp_chunks c) {
+    const int64_t s = c.start[blockIdx.x];
+    const int64_t e = s + c.len[blockIdx.x];
     double        acc = 0.0;
     if constexpr (VEC) {
         const int64_t a = min((s + 1) & ~(int64_t) 1, e), b = max(e & ~(int64_t) 1, a);
@@ -1916,15 +1907,7 @@ __global__ void __launch_bounds__(512) matvec_chunk_sums_kernel(const int32_t *_
             acc += v;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double ws[16];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double v = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    }
+    chunk_mean(c, acc);
 }
 
 // y = P x and the block means of y into N->means.  Returns MDP_EUNSUPPORTED
@@ -1936,11 +1919,9 @@ int mdp_matvec_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noi
         return MDP_EUNSUPPORTED;
     const bool vec = ((reinterpret_cast<uintptr_t>(A->values) | reinterpret_cast<uintptr_t>(d_y)) & 15) == 0;
     (vec ? matvec_chunk_sums_kernel<true> : matvec_chunk_sums_kernel<false>)<<<N->n_chunks, 512, 0, ctx->stream>>>(
-            A->off.as<int32_t>(), A->values, d_x, d_y, N->chunk_start.as<int64_t>(), N->chunk_len.as<int32_t>(),
-            N->partial.as<double>());
+            A->off.as<int32_t>(), A->values, d_x, d_y, N->chunks());
     MDP_CHECK_LAUNCH(ctx);
-    launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
-    MDP_CHECK_LAUNCH(ctx);
+    MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
     return MDP_OK;
 }
 
@@ -1981,11 +1962,9 @@ int mdp_stbmm_impl32(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d
     }
     if (!d_means) {
         if (N->n_chunks > 0) {
-            block_partial_sums<float><<<N->n_chunks, 512, 0, ctx->stream>>>(
-                    d_in, N->chunk_start.as<int64_t>(), N->chunk_len.as<int32_t>(), N->partial.as<double>());
+            block_means_kernel<float><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunks());
             MDP_CHECK_LAUNCH(ctx);
-            launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
-            MDP_CHECK_LAUNCH(ctx);
+            MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
         }
         d_means = N->means.as<double>();
     }
@@ -2000,18 +1979,6 @@ int mdp_stbmm32_batch(mdp_context *ctx, mdp_noise *N, const float *d_in, float *
     if (!N->covers_all || N->lambda == 1 || !d_means) return MDP_EUNSUPPORTED;
     MDP_TRY(mdp_noise_prepare_fp32(ctx, N));
     return launch_tiles<float>(ctx, N, N->p32, d_in, d_out, d_means, ncols, col_stride, d_active);
-}
-
-// chunks of the block-mean reduction (2048 to 65536 rows each, in block order)
-int mdp_noise_chunks(const mdp_noise *N, int *n_chunks, const int64_t **d_chunk_start, const int32_t **d_chunk_len,
-                     const int32_t **d_blk_chunk0, const int32_t **d_blk_nchunk, int *covers_all) {
-    *n_chunks = N->n_chunks;
-    *d_chunk_start = N->chunk_start.as<int64_t>();
-    *d_chunk_len = N->chunk_len.as<int32_t>();
-    *d_blk_chunk0 = N->blk_chunk0.as<int32_t>();
-    *d_blk_nchunk = N->blk_nchunk.as<int32_t>();
-    *covers_all = N->covers_all ? 1 : 0;
-    return MDP_OK;
 }
 
 // x4[q] = ((float) x[3q], (float) x[3q+1], (float) x[3q+2], 0): one aligned
@@ -2033,12 +2000,9 @@ __device__ __forceinline__ float p32_row(int32_t o, float w0, float w1, float w2
 __global__ void __launch_bounds__(512) matvec32_chunk_sums4_kernel(const int32_t *__restrict__ off,
                                                                    const float *__restrict__ w,
                                                                    const float4 *__restrict__ x4,
-                                                                   float *__restrict__ y,
-                                                                   const int64_t *__restrict__ chunk_start,
-                                                                   const int32_t *__restrict__ chunk_len,
-                                                                   double *__restrict__ partial) {
-    const int64_t s = chunk_start[blockIdx.x];
-    const int64_t e = s + chunk_len[blockIdx.x];
+                                                                   float *__restrict__ y, mdp_chunks c) {
+    const int64_t s = c.start[blockIdx.x];
+    const int64_t e = s + c.len[blockIdx.x];
     const int64_t a = min((s + 3) & ~(int64_t) 3, e);  // first multiple of 4 in [s, e]
     const int64_t b = max(e & ~(int64_t) 3, a);         // end of the aligned body
     double        acc = 0.0;
@@ -2062,26 +2026,15 @@ __global__ void __launch_bounds__(512) matvec32_chunk_sums4_kernel(const int32_t
         y[t] = v;
         acc += (double) v;
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double wsum[16];
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double v = (threadIdx.x < (blockDim.x >> 5)) ? wsum[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    }
+    chunk_mean(c, acc);
 }
 
 // y32 = P x (x FP64, weights FP32) fused with FP64 block-mean partial sums
 __global__ void __launch_bounds__(512) matvec32_chunk_sums_kernel(const int32_t *__restrict__ off,
                                                                   const float *__restrict__ w,
-                                                                  const double *__restrict__ x, float *__restrict__ y,
-                                                                  const int64_t *__restrict__ chunk_start,
-                                                                  const int32_t *__restrict__ chunk_len,
-                                                                  double *__restrict__ partial) {
-    const int64_t s = chunk_start[blockIdx.x];
-    const int     n = chunk_len[blockIdx.x];
+                                                                  const double *__restrict__ x, float *__restrict__ y, mdp_chunks c) {
+    const int64_t s = c.start[blockIdx.x];
+    const int     n = c.len[blockIdx.x];
     double        acc = 0.0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         const int64_t t = s + j;
@@ -2093,15 +2046,7 @@ __global__ void __launch_bounds__(512) matvec32_chunk_sums_kernel(const int32_t 
         y[t] = v;
         acc += (double) v;
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double ws[16];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double v = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    }
+    chunk_mean(c, acc);
 }
 
 int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noise *N, const double *d_x,
@@ -2118,16 +2063,13 @@ int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_n
         map_to_float4_kernel<<<grid_for(npix, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(d_x, x4, npix);
         MDP_CHECK_LAUNCH(ctx);
         matvec32_chunk_sums4_kernel<<<N->n_chunks, 512, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->w32.as<float>(), x4, d_y, N->chunk_start.as<int64_t>(),
-                N->chunk_len.as<int32_t>(), N->partial.as<double>());
+                A->off.as<int32_t>(), A->w32.as<float>(), x4, d_y, N->chunks());
     } else {
         matvec32_chunk_sums_kernel<<<N->n_chunks, 512, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->w32.as<float>(), d_x, d_y, N->chunk_start.as<int64_t>(),
-                N->chunk_len.as<int32_t>(), N->partial.as<double>());
+                A->off.as<int32_t>(), A->w32.as<float>(), d_x, d_y, N->chunks());
     }
     MDP_CHECK_LAUNCH(ctx);
-    launch_means_final(ctx, N, N->partial.as<double>(), N->means.as<double>());
-    MDP_CHECK_LAUNCH(ctx);
+    MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
     return MDP_OK;
 }
 
@@ -2280,11 +2222,9 @@ extern "C" int mdp_stbmm_noalloc(mdp_context *ctx, const mdp_noise *N, const dou
     double *partial = scratch;                 // [n_chunks], each written before it is read
     double *means = scratch + N->n_chunks;     // [nb], each written before it is read
     if (N->n_chunks > 0) {
-        block_partial_sums<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunk_start.as<int64_t>(),
-                                                                 N->chunk_len.as<int32_t>(), partial);
+        block_means_kernel<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunks(partial, means));
         MDP_CHECK_LAUNCH(ctx);
-        launch_means_final(ctx, N, partial, means);
-        MDP_CHECK_LAUNCH(ctx);
+        MDP_TRY(mdp_means_final(ctx, N, N->chunks(partial, means), 1));
     } else {
         MDP_CUDA(cudaMemsetAsync(means, 0, sizeof(double) * N->nb, ctx->stream));
     }

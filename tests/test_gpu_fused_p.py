@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("sizes,tail", [([1], 0), ([2, 1, 3, 1], 0), ([2047, 2049, 1, 4098, 2], 0), ([4096, 2048, 6145], 0),
+@pytest.mark.parametrize("sizes,tail", [([1], 0), ([2000] * 70 + [65537] * 30, 5), ([2, 1, 3, 1], 0), ([2047, 2049, 1, 4098, 2], 0), ([4096, 2048, 6145], 0),
                                         ([500, 700], 333)])   # rows past the last block pass through N^-1
 def test_operator_over_chunk_edges(gpu_ctx, sizes, tail, shift):
     import torch
