@@ -605,6 +605,8 @@ __global__ void __launch_bounds__(256) matvec_triplet_kernel(const int32_t *__re
                                                              const double *__restrict__ w,
                                                              const double *__restrict__ x, double *__restrict__ y,
                                                              int64_t m) {
+    chain_next();
+    chain_wait();
     const int64_t npair = m >> 1;
     for (int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; p < npair; p += (int64_t) gridDim.x * blockDim.x) {
         const int2    o  = reinterpret_cast<const int2 *>(off)[p];
@@ -612,14 +614,14 @@ __global__ void __launch_bounds__(256) matvec_triplet_kernel(const int32_t *__re
         const double2 b  = reinterpret_cast<const double2 *>(w)[3 * p + 1];
         const double2 c  = reinterpret_cast<const double2 *>(w)[3 * p + 2];
         double        y0 = 0.0, y1 = 0.0;
-        if (o.x >= 0) y0 = a.x * __ldg(x + o.x) + a.y * __ldg(x + o.x + 1) + b.x * __ldg(x + o.x + 2);
-        if (o.y >= 0) y1 = b.y * __ldg(x + o.y) + c.x * __ldg(x + o.y + 1) + c.y * __ldg(x + o.y + 2);
+        if (o.x >= 0) y0 = a.x * ld_after(x + o.x) + a.y * ld_after(x + o.x + 1) + b.x * ld_after(x + o.x + 2);
+        if (o.y >= 0) y1 = b.y * ld_after(x + o.y) + c.x * ld_after(x + o.y + 1) + c.y * ld_after(x + o.y + 2);
         reinterpret_cast<double2 *>(y)[p] = make_double2(y0, y1);
     }
     if ((m & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
         int64_t t = m - 1;
         int32_t o = off[t];
-        y[t]      = (o >= 0) ? w[3 * t] * x[o] + w[3 * t + 1] * x[o + 1] + w[3 * t + 2] * x[o + 2] : 0.0;
+        y[t]      = (o >= 0) ? w[3 * t] * ld_after(x + o) + w[3 * t + 1] * ld_after(x + o + 1) + w[3 * t + 2] * ld_after(x + o + 2) : 0.0;
     }
 }
 
@@ -670,8 +672,8 @@ int mdp_matvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d_x
                 A->off.as<int32_t>(), A->values, d_x, d_y, A->m);
     } else if (A->triplet) {
         int64_t npair = A->m >> 1;
-        matvec_triplet_kernel<<<grid_for(npair > 0 ? npair : 1, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->values, d_x, d_y, A->m);
+        MDP_CUDA(launch_chained(matvec_triplet_kernel, grid_for(npair > 0 ? npair : 1, 256, ctx->sm_count * 16), 256, 0,
+                                ctx->stream, A->off.as<int32_t>(), A->values, d_x, d_y, A->m));
     } else {
         matvec_general_kernel<<<grid_for(A->m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
                 A->local.as<int32_t>(), A->values, d_x, d_y, A->m, A->nnz, A->trash_pix);
@@ -686,15 +688,23 @@ extern "C" int mdp_matvec(mdp_context *ctx, const mdp_pointing *A, const double 
 }
 
 // ============================================================== x = P^T y
+__global__ void pt_zero_kernel(double *__restrict__ x, int64_t n) {
+    chain_next();
+    chain_wait();
+    for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) x[i] = 0.0;
+}
+
 // FP64 atomics into the (L2-resident) map.
 __global__ void __launch_bounds__(256) trmatvec_triplet_kernel(const int32_t *__restrict__ off,
                                                                const double *__restrict__ w,
                                                                const double *__restrict__ y, double *__restrict__ x,
                                                                int64_t m) {
+    chain_next();
+    chain_wait();
     const int64_t npair = m >> 1;
     for (int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; p < npair; p += (int64_t) gridDim.x * blockDim.x) {
         const int2    o  = reinterpret_cast<const int2 *>(off)[p];
-        const double2 yy = reinterpret_cast<const double2 *>(y)[p];
+        const double2 yy = ld_after(reinterpret_cast<const double2 *>(y) + p);
         const double2 a  = reinterpret_cast<const double2 *>(w)[3 * p];
         const double2 b  = reinterpret_cast<const double2 *>(w)[3 * p + 1];
         const double2 c  = reinterpret_cast<const double2 *>(w)[3 * p + 2];
@@ -713,7 +723,7 @@ __global__ void __launch_bounds__(256) trmatvec_triplet_kernel(const int32_t *__
         int64_t t = m - 1;
         int32_t o = off[t];
         if (o >= 0)
-            for (int j = 0; j < 3; j++) atomicAdd(x + o + j, w[3 * t + j] * y[t]);
+            for (int j = 0; j < 3; j++) atomicAdd(x + o + j, w[3 * t + j] * ld_after(y + t));
     }
 }
 
@@ -1005,6 +1015,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
     const int     wid = threadIdx.x >> 5, lane = lane_id();
     const int64_t sl = (int64_t) blockIdx.x * PT_WARPS + wid;
     const int     out = group_out[blockIdx.x];  // -2: a bin a warp; -1: one bin; else the row of `partial`
+    chain_next();
     if (sl >= nslices) return;  // whole warps, only of the last group of kind -2: no barrier follows there
     double *acc = acc_s[wid];
     for (int i = lane; i < 3 * PT_BIN_PIX; i += 32) acc[i] = 0.0;
@@ -1012,6 +1023,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
     const int64_t bin = slice_bin[sl];
     const int64_t s0 = slice_lo[sl], s1 = slice_hi[sl];
     const int64_t base = bin * 3 * PT_BIN_PIX;
+    chain_wait();
     // the row numbers of the next U steps are loaded while the current ones are
     // gathered and added: one memory latency per U steps on the warp's path
     uint32_t tn[U];
@@ -1039,7 +1051,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
             c0[u] = c1[u] = c2[u] = 0.0;
             if (o[u] >= 0) {
                 const int64_t t = tc[u];
-                const double  v = (double) y[t];
+                const double  v = (double) ld_after(y + t);
                 c0[u] = (double) w[3 * t] * v;
                 c1[u] = (double) w[3 * t + 1] * v;
                 c2[u] = (double) w[3 * t + 2] * v;
@@ -1112,6 +1124,8 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 4) trmatvec_slices_kernel(
 __global__ void pt_partial_sum_kernel(const double *__restrict__ partial, const int32_t *__restrict__ multi_bin,
                                       const int32_t *__restrict__ multi_first, const int32_t *__restrict__ multi_n,
                                       int64_t nmulti, double *__restrict__ x, int64_t n_map) {
+    chain_next();
+    chain_wait();
     constexpr int E = 3 * PT_BIN_PIX;
     for (int64_t idx = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; idx < nmulti * E;
          idx += (int64_t) gridDim.x * blockDim.x) {
@@ -1120,7 +1134,7 @@ __global__ void pt_partial_sum_kernel(const double *__restrict__ partial, const 
         if (xi >= n_map) continue;
         const double *pr = partial + (int64_t) multi_first[k] * E + e;
         double        s = 0.0;
-        for (int j = 0; j < multi_n[k]; j++) s += pr[(int64_t) j * E];
+        for (int j = 0; j < multi_n[k]; j++) s += ld_after(pr + (int64_t) j * E);
         x[xi] = s;
     }
 }
@@ -1130,17 +1144,17 @@ template <typename TY, typename TW>
 static int trmatvec_slices(mdp_context *ctx, const mdp_pointing *A, const TW *w, const TY *d_y, double *d_x) {
     const mdp_pt_bins &B = A->bins;
     if (B.nslices > 0) {
-        trmatvec_slices_kernel<TY, TW><<<(unsigned) ((B.nslices + PT_WARPS - 1) / PT_WARPS), 32 * PT_WARPS, 0,
-                                         ctx->stream>>>(
+        MDP_CUDA(launch_chained(
+                trmatvec_slices_kernel<TY, TW>, (unsigned) ((B.nslices + PT_WARPS - 1) / PT_WARPS), 32 * PT_WARPS, 0, ctx->stream,
                 w, d_y, d_x, B.perm.as<uint32_t>(), B.pix.as<uint8_t>(), B.slice_bin.as<int32_t>(),
                 B.slice_lo.as<uint32_t>(), B.slice_hi.as<uint32_t>(), B.group_out.as<int32_t>(), B.nslices,
-                B.partial.as<double>(), A->n_map());
+                B.partial.as<double>(), A->n_map()));
         MDP_CHECK_LAUNCH(ctx);
     }
     if (B.nmulti > 0) {
-        pt_partial_sum_kernel<<<grid_for(B.nmulti * 3 * PT_BIN_PIX, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
-                B.partial.as<double>(), B.multi_bin.as<int32_t>(), B.multi_first.as<int32_t>(),
-                B.multi_n.as<int32_t>(), B.nmulti, d_x, A->n_map());
+        MDP_CUDA(launch_chained(pt_partial_sum_kernel, grid_for(B.nmulti * 3 * PT_BIN_PIX, 256, ctx->sm_count * 8), 256, 0,
+                                ctx->stream, B.partial.as<double>(), B.multi_bin.as<int32_t>(),
+                                B.multi_first.as<int32_t>(), B.multi_n.as<int32_t>(), B.nmulti, d_x, A->n_map()));
         MDP_CHECK_LAUNCH(ctx);
     }
     return MDP_OK;
@@ -1190,14 +1204,15 @@ int mdp_trmatvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d
         // every map entry is written by its bin's slice or by the partial sums
         return trmatvec_slices<double, double>(ctx, A, A->values, d_y, d_x);
     }
-    MDP_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * A->n_map(), ctx->stream));
+    MDP_CUDA(launch_chained(pt_zero_kernel, grid_for(A->n_map(), 256, ctx->sm_count * 8), 256, 0, ctx->stream, d_x, A->n_map()));
+    MDP_CHECK_LAUNCH(ctx);
     if (A->triplet && !aligned16(A->values, d_y)) {
         trmatvec_triplet_scalar_kernel<<<grid_for(A->m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
                 A->off.as<int32_t>(), A->values, d_y, d_x, A->m);
     } else if (A->triplet) {
         int64_t npair = A->m >> 1;
-        trmatvec_triplet_kernel<<<grid_for(npair > 0 ? npair : 1, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->values, d_y, d_x, A->m);
+        MDP_CUDA(launch_chained(trmatvec_triplet_kernel, grid_for(npair > 0 ? npair : 1, 256, ctx->sm_count * 16), 256, 0,
+                                ctx->stream, A->off.as<int32_t>(), A->values, d_y, d_x, A->m));
     } else {
         trmatvec_general_kernel<<<grid_for(A->m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
                 A->local.as<int32_t>(), A->values, d_y, d_x, A->m, A->nnz, A->trash_pix);

@@ -108,7 +108,7 @@ template <typename T>
 __device__ __forceinline__ bool tile_of(const RArgs<T> &a, int64_t item, Tile<T> &tl, int &spec) {
     const uint32_t col = item < a.n_tiles ? 0u : (uint32_t) item / (uint32_t) a.n_tiles;
     const int64_t  tile = item - col * a.n_tiles;
-    if (a.active && !a.active[col]) return false;
+    chain_next();
     const int4 d0 = __ldg(reinterpret_cast<const int4 *>(a.tiles + tile)), d1 = __ldg(reinterpret_cast<const int4 *>(a.tiles + tile) + 1);
     const int64_t bs = (int64_t) (((uint64_t) (uint32_t) d0.y << 32) | (uint32_t) d0.x) + col * a.col_stride;
     tl.in = a.vin + bs;
@@ -117,11 +117,13 @@ __device__ __forceinline__ bool tile_of(const RArgs<T> &a, int64_t item, Tile<T>
     tl.len = d0.w;
     tl.e = d1.x;
     spec = d1.y;
+    chain_wait();  // the records above are the plan's own; all else may come from the kernel before
+    if (a.active && !a.active[col]) return false;
     tl.mu = a.means ? (T) a.means[col * a.nb + d1.z] : (T) 0;
     return true;
 }
 
-__device__ __forceinline__ float ld_stream(const float *p) {  // read once: not kept in L1
+__device__ __forceinline__ float ld_stream(const float *p) {  // constant, read once: not kept in L1
     float v;
     asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
@@ -131,16 +133,26 @@ __device__ __forceinline__ double ld_stream(const double *p) {
     asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
+__device__ __forceinline__ float ld_sample(const float *p) {  // from the kernel before (as ld_after), read once
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_sample(const double *p) {
+    double v;
+    asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 // sample n of the window, less the block mean; zero outside the block
 template <typename T>
 __device__ __forceinline__ T sample(const Tile<T> &tl, int n) {
     const int i = tl.o + n;
-    return (unsigned) i < (unsigned) tl.len ? ld_stream(tl.in + i) - tl.mu : (T) 0;
+    return (unsigned) i < (unsigned) tl.len ? ld_sample(tl.in + i) - tl.mu : (T) 0;
 }
 // the same of a window inside its block: point j0 + n, n known at compile time
 template <typename T>
 __device__ __forceinline__ T sample_in(const Tile<T> &tl, int j0, int n) {
-    return ld_stream(tl.in + (tl.o + j0) + n) - tl.mu;
+    return ld_sample(tl.in + (tl.o + j0) + n) - tl.mu;
 }
 __device__ __forceinline__ double sample(const RowSrc &r, int n) {
     return n < r.lambda ? __ldg(r.T + n) : (r.M2 - n < r.lambda ? -__ldg(r.T + (r.M2 - n)) : 0.0);
@@ -193,13 +205,15 @@ template <typename G> __device__ __forceinline__ CP<G> get(const REnt<G> *p) {
     const REnt<G> e = *p;
     return {e.x, e.y};
 }
-// from L2, where other CTAs wrote it
+// from L2, where the kernel before wrote it
 __device__ __forceinline__ CP<mono32> get_l2(const REnt<mono32> *p) {
-    const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return {Pr<mono32>{v.x}, Pr<mono32>{v.y}};
 }
 __device__ __forceinline__ CP<mono64> get_l2(const REnt<mono64> *p) {
-    const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+    double2 v;
+    asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
     return {Pr<mono64>{v.x}, Pr<mono64>{v.y}};
 }
 
@@ -654,29 +668,35 @@ int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, c
     const int64_t items = P.n_tiles * ncols;
     if (items << P.log_m1 > 0x7fffffffLL) return MDP_EUNSUPPORTED;
     void *args[] = {&a};
-    if (m1 == 1) {
-        MDP_CUDA(cudaLaunchKernel(one_fn<T>(L), dim3((unsigned) items), dim3(L / 16), args, rows_smem<T>(L), ctx->stream));
+    // Chained to the kernel before, but for the first launches of two streams; FP64 groups on two
+    // streams are not: a waiting CTA takes one of an SM's two places from the other stream's group
+    // (64 x 2^20 samples, half bandwidth 2^14: 1.206 against 1.194 ms; FP32, of four places, 0.647 ->
+    // 0.620 ms, and one group 140 -> 129 us for 24 ragged blocks).
+    auto launch = [&](const void *fn, dim3 grid, int nt, size_t smem, cudaStream_t stream, bool chain) -> int {
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t  cfg = chained_config(&attr, stream, grid, nt, smem);
+        if (!chain) cfg.numAttrs = 0;
+        MDP_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
         MDP_CHECK_LAUNCH(ctx);
         return MDP_OK;
-    }
+    };
+    if (m1 == 1) return launch(one_fn<T>(L), dim3((unsigned) items), L / 16, rows_smem<T>(L), ctx->stream, true);
     const Groups g = groups_of(items, 2 * (int64_t) sizeof(T) * M, (int64_t) P.scratch.bytes);
     cudaStream_t st[2] = {ctx->stream, ctx->stream};
     if (g.n > 1) {
         MDP_TRY(mdp_side_fork(ctx));
         st[1] = ctx->side;
     }
-    auto *Y = a.Y;
+    auto      *Y = a.Y;
+    const bool chain = sizeof(T) == 4 || g.n == 1;
     for (int64_t k = 0; k < g.n; k++) {
         const int64_t i = k * g.per;
         const dim3    grid((unsigned) (std::min(g.per, items - i) * m1));
         a.item0 = i;
         a.Y = Y + (k & 1) * g.per * M;
-        MDP_CUDA(cudaLaunchKernel(cols_fn<T, false>(P.log_m1), grid, dim3(256), args, 0, st[k & 1]));
-        MDP_CHECK_LAUNCH(ctx);
-        MDP_CUDA(cudaLaunchKernel((const void *) rt_rows_kernel<T>, grid, dim3(256), args, rows_smem<T>(L), st[k & 1]));
-        MDP_CHECK_LAUNCH(ctx);
-        MDP_CUDA(cudaLaunchKernel(cols_fn<T, true>(P.log_m1), grid, dim3(256), args, 0, st[k & 1]));
-        MDP_CHECK_LAUNCH(ctx);
+        MDP_TRY(launch(cols_fn<T, false>(P.log_m1), grid, 256, 0, st[k & 1], g.n == 1 || (chain && k > 1)));
+        MDP_TRY(launch((const void *) rt_rows_kernel<T>, grid, 256, rows_smem<T>(L), st[k & 1], chain));
+        MDP_TRY(launch(cols_fn<T, true>(P.log_m1), grid, 256, 0, st[k & 1], chain));
     }
     if (g.n > 1) MDP_TRY(mdp_side_join(ctx));
     return MDP_OK;

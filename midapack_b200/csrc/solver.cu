@@ -535,9 +535,11 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_init_kernel(const double *__r
 // coeff = (h, AtNm1Ah)
 __global__ void __launch_bounds__(RED_THREADS) pcg_coeff_kernel(const double *__restrict__ h,
                                                                 const double *__restrict__ q_, int64_t n, Scal *S) {
+    chain_next();
+    chain_wait();
     double v[1] = {0.0};
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
-        v[0] += h[i] * q_[i];
+        v[0] += ld_after(h + i) * ld_after(q_ + i);
     block_reduce_store<1>(v, S, 0);
     if (last_block(S, 1)) {
         const double *t = sum_partials<1>(S);
@@ -554,6 +556,8 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_update_kernel(const double *_
                                                                  const double *__restrict__ q_,
                                                                  const double *__restrict__ gp, double *__restrict__ g,
                                                                  double *__restrict__ Cg, int64_t npix, Scal *S) {
+    chain_next();
+    chain_wait();
     const double ro = S->ro;
     double       v[3] = {0.0, 0.0, 0.0};
     for (int64_t q = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += (int64_t) gridDim.x * blockDim.x) {
@@ -561,9 +565,9 @@ __global__ void __launch_bounds__(RED_THREADS) pcg_update_kernel(const double *_
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             const int64_t i = 3 * q + j;
-            x[i] = x[i] + ro * h[i];
-            go[j] = gp[i];
-            gn[j] = go[j] - ro * q_[i];
+            x[i] = x[i] + ro * ld_after(h + i);
+            go[j] = ld_after(gp + i);
+            gn[j] = go[j] - ro * ld_after(q_ + i);
             g[i] = gn[j];
         }
         const double *I = inv + 9 * q;
@@ -730,9 +734,11 @@ __global__ void __launch_bounds__(RED_THREADS) dot_self_kernel(const double *__r
 
 // h = gamma h + Cg
 __global__ void pcg_direction_kernel(double *__restrict__ h, const double *__restrict__ Cg, int64_t n, const Scal *S) {
+    chain_next();
+    chain_wait();
     const double gamma = S->gamma;
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
-        h[i] = h[i] * gamma + Cg[i];
+        h[i] = h[i] * gamma + ld_after(Cg + i);
 }
 
 // rows past the last noise block: N^-1 leaves them as they are (mdp_stbmm writes the rows up
@@ -901,7 +907,7 @@ int mdp_pcg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
         if (prof) cudaEventRecord(ctx->ev[2], st);
         MDP_TRY(mdp_trmatvec_launch(ctx, A, tb, q));
         if (prof) cudaEventRecord(ctx->ev[3], st);
-        pcg_coeff_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(h, q, n, S);
+        MDP_CUDA(launch_chained(pcg_coeff_kernel, RED_BLOCKS, RED_THREADS, 0, st, h, q, n, S));
         MDP_CHECK_LAUNCH(ctx);
         if (tl) {
             pcg_step_kernel<<<grid_for(n, 256, ctx->sm_count * 8), 256, 0, st>>>(x, h, q, gp, g, n, S);
@@ -911,7 +917,7 @@ int mdp_pcg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
                                                                       tl->AZ.as<double>(), tl->qtx.as<double>(),
                                                                       tl->zn, S);
         } else {
-            pcg_update_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(inv, x, h, q, gp, g, Cg, npix, S);
+            MDP_CUDA(launch_chained(pcg_update_kernel, RED_BLOCKS, RED_THREADS, 0, st, inv, x, h, q, gp, g, Cg, npix, S));
         }
         MDP_CHECK_LAUNCH(ctx);
         if (prof) cudaEventRecord(ctx->ev[4], st);
@@ -1148,7 +1154,7 @@ extern "C" int mdp_gls_solve_mixed(mdp_context *ctx, mdp_pointing *A, const mdp_
             if (prof) cudaEventRecord(ctx->ev[2], st);
             MDP_TRY(mdp_trmatvec32_launch(ctx, A, fb, q));
             if (prof) cudaEventRecord(ctx->ev[3], st);
-            pcg_coeff_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(h, q, n, S);
+            MDP_CUDA(launch_chained(pcg_coeff_kernel, RED_BLOCKS, RED_THREADS, 0, st, h, q, n, S));
             MDP_CHECK_LAUNCH(ctx);
             if (tl) {
                 pcg_step_kernel<<<grid_for(n, 256, ctx->sm_count * 8), 256, 0, st>>>(dl, h, q, gp, g, n, S);
@@ -1158,7 +1164,7 @@ extern "C" int mdp_gls_solve_mixed(mdp_context *ctx, mdp_pointing *A, const mdp_
                                                                           tl->AZ.as<double>(), tl->qtx.as<double>(),
                                                                           tl->zn, S);
             } else {
-                pcg_update_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(inv, dl, h, q, gp, g, Cg, npix, S);
+                MDP_CUDA(launch_chained(pcg_update_kernel, RED_BLOCKS, RED_THREADS, 0, st, inv, dl, h, q, gp, g, Cg, npix, S));
             }
             MDP_CHECK_LAUNCH(ctx);
             if (prof) cudaEventRecord(ctx->ev[4], st);

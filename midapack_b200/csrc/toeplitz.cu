@@ -1036,28 +1036,32 @@ static size_t tile_smem(int log_ml) {
 // ------------------------------------------------------------------ block means and white noise
 template <typename T>
 __global__ void __launch_bounds__(512) block_means_kernel(const T *__restrict__ v, mdp_chunks c) {
+    chain_next();
+    chain_wait();
     const int64_t s = c.start[blockIdx.x];
     const int     n = c.len[blockIdx.x];
     double        acc = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) acc += (double) v[s + j];
+    for (int j = threadIdx.x; j < n; j += blockDim.x) acc += (double) ld_after(v + s + j);
     chunk_mean(c, acc);
 }
 
 // the mean of every block from its chunk sums, a warp a block, column blockIdx.y of a batch
 __global__ void block_means_final(mdp_chunks c, int n_chunks, int nb) {
+    chain_next();
+    chain_wait();
     const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
     for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nw) {
         const int     n = c.blk_nchunk[b];
         const double *p = c.partial + (int64_t) blockIdx.y * n_chunks + c.blk_chunk0[b];
         double        s = 0.0;
-        for (int i = lane; i < n; i += 32) s += p[i];
+        for (int i = lane; i < n; i += 32) s += ld_after(p + i);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) c.means[(int64_t) blockIdx.y * nb + b] = s / (double) c.blk_len[b];
     }
 }
 int mdp_means_final(mdp_context *ctx, const mdp_noise *N, const mdp_chunks &c, int ncols) {
     if (c.arrived) return MDP_OK;  // taken by the chunks' kernel
-    block_means_final<<<dim3(grid_for(N->nb, 4, 2048), ncols), 128, 0, ctx->stream>>>(c, N->n_chunks, N->nb);
+    MDP_CUDA(launch_chained(block_means_final, dim3(grid_for(N->nb, 4, 2048), ncols), 128, 0, ctx->stream, c, N->n_chunks, N->nb));
     MDP_CHECK_LAUNCH(ctx);
     return MDP_OK;
 }
@@ -1843,7 +1847,7 @@ int mdp_block_means(mdp_context *ctx, const mdp_noise *N, const double *d_v, dou
         return MDP_OK;
     }
     const mdp_chunks c = N->chunks(N->partial.as<double>(), d_means);
-    block_means_kernel<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_v, c);
+    MDP_CUDA(launch_chained(block_means_kernel<double>, N->n_chunks, 512, 0, ctx->stream, d_v, c));
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(mdp_means_final(ctx, N, c, 1));
     return MDP_OK;
@@ -1873,13 +1877,15 @@ int mdp_stbmm_impl(mdp_context *ctx, const mdp_noise *N, const double *d_in, dou
 // the chunk's odd first and last row by themselves).  Bound: DRAM.  With one row a thread and
 // fixed chunks of 65536 rows, 4 x 2^20 rows ran on 64 CTAs and took 138 us.
 __device__ __forceinline__ double p64_row(int32_t o, double w0, double w1, double w2, const double *__restrict__ x) {
-    return o >= 0 ? w0 * __ldg(x + o) + w1 * __ldg(x + o + 1) + w2 * __ldg(x + o + 2) : 0.0;
+    return o >= 0 ? w0 * ld_after(x + o) + w1 * ld_after(x + o + 1) + w2 * ld_after(x + o + 2) : 0.0;
 }
 template <bool VEC>
 __global__ void __launch_bounds__(512) matvec_chunk_sums_kernel(const int32_t *__restrict__ off,
                                                                 const double *__restrict__ w,
                                                                 const double *__restrict__ x, double *__restrict__ y,
                                                                 mdp_chunks c) {
+    chain_next();
+    chain_wait();
     const int64_t s = c.start[blockIdx.x];
     const int64_t e = s + c.len[blockIdx.x];
     double        acc = 0.0;
@@ -1918,8 +1924,8 @@ int mdp_matvec_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_noi
     if (!A->triplet || !N->covers_all || N->lambda == 1 || N->nrow_end != A->m || N->n_chunks == 0)
         return MDP_EUNSUPPORTED;
     const bool vec = ((reinterpret_cast<uintptr_t>(A->values) | reinterpret_cast<uintptr_t>(d_y)) & 15) == 0;
-    (vec ? matvec_chunk_sums_kernel<true> : matvec_chunk_sums_kernel<false>)<<<N->n_chunks, 512, 0, ctx->stream>>>(
-            A->off.as<int32_t>(), A->values, d_x, d_y, N->chunks());
+    MDP_CUDA(launch_chained(vec ? matvec_chunk_sums_kernel<true> : matvec_chunk_sums_kernel<false>, N->n_chunks, 512, 0,
+                            ctx->stream, A->off.as<int32_t>(), A->values, d_x, d_y, N->chunks()));
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
     return MDP_OK;
@@ -1962,7 +1968,7 @@ int mdp_stbmm_impl32(mdp_context *ctx, mdp_noise *N, const float *d_in, float *d
     }
     if (!d_means) {
         if (N->n_chunks > 0) {
-            block_means_kernel<float><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunks());
+            MDP_CUDA(launch_chained(block_means_kernel<float>, N->n_chunks, 512, 0, ctx->stream, d_in, N->chunks()));
             MDP_CHECK_LAUNCH(ctx);
             MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
         }
@@ -1984,13 +1990,15 @@ int mdp_stbmm32_batch(mdp_context *ctx, mdp_noise *N, const float *d_in, float *
 // x4[q] = ((float) x[3q], (float) x[3q+1], (float) x[3q+2], 0): one aligned
 // 16-byte gather per sample in the FP32 P instead of three 8-byte ones
 __global__ void map_to_float4_kernel(const double *__restrict__ x, float4 *__restrict__ x4, int64_t npix) {
+    chain_next();
+    chain_wait();
     for (int64_t q = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += (int64_t) gridDim.x * blockDim.x)
-        x4[q] = make_float4((float) x[3 * q], (float) x[3 * q + 1], (float) x[3 * q + 2], 0.0f);
+        x4[q] = make_float4((float) ld_after(x + 3 * q), (float) ld_after(x + 3 * q + 1), (float) ld_after(x + 3 * q + 2), 0.0f);
 }
 
 __device__ __forceinline__ float p32_row(int32_t o, float w0, float w1, float w2, const float4 *__restrict__ x4) {
     if (o < 0) return 0.0f;
-    const float4 m = __ldg(x4 + o / 3);
+    const float4 m = ld_after(x4 + o / 3);
     return w0 * m.x + w1 * m.y + w2 * m.z;
 }
 
@@ -2001,6 +2009,8 @@ __global__ void __launch_bounds__(512) matvec32_chunk_sums4_kernel(const int32_t
                                                                    const float *__restrict__ w,
                                                                    const float4 *__restrict__ x4,
                                                                    float *__restrict__ y, mdp_chunks c) {
+    chain_next();
+    chain_wait();
     const int64_t s = c.start[blockIdx.x];
     const int64_t e = s + c.len[blockIdx.x];
     const int64_t a = min((s + 3) & ~(int64_t) 3, e);  // first multiple of 4 in [s, e]
@@ -2033,6 +2043,8 @@ __global__ void __launch_bounds__(512) matvec32_chunk_sums4_kernel(const int32_t
 __global__ void __launch_bounds__(512) matvec32_chunk_sums_kernel(const int32_t *__restrict__ off,
                                                                   const float *__restrict__ w,
                                                                   const double *__restrict__ x, float *__restrict__ y, mdp_chunks c) {
+    chain_next();
+    chain_wait();
     const int64_t s = c.start[blockIdx.x];
     const int     n = c.len[blockIdx.x];
     double        acc = 0.0;
@@ -2041,8 +2053,8 @@ __global__ void __launch_bounds__(512) matvec32_chunk_sums_kernel(const int32_t 
         const int32_t o = off[t];
         float         v = 0.0f;
         if (o >= 0)
-            v = w[3 * t] * (float) __ldg(x + o) + w[3 * t + 1] * (float) __ldg(x + o + 1) +
-                w[3 * t + 2] * (float) __ldg(x + o + 2);
+            v = w[3 * t] * (float) ld_after(x + o) + w[3 * t + 1] * (float) ld_after(x + o + 1) +
+                w[3 * t + 2] * (float) ld_after(x + o + 2);
         y[t] = v;
         acc += (double) v;
     }
@@ -2060,13 +2072,14 @@ int mdp_matvec32_blockmeans(mdp_context *ctx, const mdp_pointing *A, const mdp_n
     if (vec) {
         MDP_TRY(ctx->ws[12].alloc(sizeof(float4) * (size_t) std::max<int64_t>(npix, 1)));
         float4 *x4 = ctx->ws[12].as<float4>();
-        map_to_float4_kernel<<<grid_for(npix, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(d_x, x4, npix);
+        MDP_CUDA(launch_chained(map_to_float4_kernel, grid_for(npix, 256, ctx->sm_count * 8), 256, 0, ctx->stream, d_x, x4,
+                                npix));
         MDP_CHECK_LAUNCH(ctx);
-        matvec32_chunk_sums4_kernel<<<N->n_chunks, 512, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->w32.as<float>(), x4, d_y, N->chunks());
+        MDP_CUDA(launch_chained(matvec32_chunk_sums4_kernel, N->n_chunks, 512, 0, ctx->stream, A->off.as<int32_t>(),
+                                A->w32.as<float>(), x4, d_y, N->chunks()));
     } else {
-        matvec32_chunk_sums_kernel<<<N->n_chunks, 512, 0, ctx->stream>>>(
-                A->off.as<int32_t>(), A->w32.as<float>(), d_x, d_y, N->chunks());
+        MDP_CUDA(launch_chained(matvec32_chunk_sums_kernel, N->n_chunks, 512, 0, ctx->stream, A->off.as<int32_t>(),
+                                A->w32.as<float>(), d_x, d_y, N->chunks()));
     }
     MDP_CHECK_LAUNCH(ctx);
     MDP_TRY(mdp_means_final(ctx, N, N->chunks(), 1));
@@ -2222,7 +2235,7 @@ extern "C" int mdp_stbmm_noalloc(mdp_context *ctx, const mdp_noise *N, const dou
     double *partial = scratch;                 // [n_chunks], each written before it is read
     double *means = scratch + N->n_chunks;     // [nb], each written before it is read
     if (N->n_chunks > 0) {
-        block_means_kernel<double><<<N->n_chunks, 512, 0, ctx->stream>>>(d_in, N->chunks(partial, means));
+        MDP_CUDA(launch_chained(block_means_kernel<double>, N->n_chunks, 512, 0, ctx->stream, d_in, N->chunks(partial, means)));
         MDP_CHECK_LAUNCH(ctx);
         MDP_TRY(mdp_means_final(ctx, N, N->chunks(partial, means), 1));
     } else {
