@@ -28,15 +28,15 @@
 // values with real and imaginary parts exchanged, conj(DFT(conj v)) =
 // swap(DFT(swap v)), a renaming of registers.
 //
-// One tile a CTA (FP32: 16 points take 32 of 64 registers, four CTAs of 256 threads an SM;
+// One tile a CTA (FP32: 16 points take 32 of 80 registers, three CTAs of 256 threads an SM;
 // FP64: 64 of 128, two).  FP32 complex sums are one paired FP32 instruction (add/sub
 // .f32x2) on (x, y).  Two FP32 tiles on the lanes of paired instructions took fewer
 // instructions and half the resident warps: 0.71 against 0.70 ms below, 131 against 94 us for
 // 8 x 2^20 samples at half bandwidth 2^13.
 //
 // Measured against the best of the even/odd-packed plans on a B200 (64 x 2^20 samples,
-// half bandwidth 2^14): FP32 0.93 -> 0.645 ms, error against 64 bits 5.9e-7 -> 2.7e-7; FP64
-// 1.62 -> 1.20 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 76 % busy in
+// half bandwidth 2^14): FP32 0.93 -> 0.58 ms, error against 64 bits 5.9e-7 -> 2.7e-7; FP64
+// 1.62 -> 1.19 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 76 % busy in
 // FP32, waiting for its loads in FP64.  A spectrum from the transform itself takes
 // microseconds where the direct cosine sums took 3.7 ms (half bandwidth 2^13, 2^17 samples).
 #include <algorithm>
@@ -86,8 +86,9 @@ struct RArgs {
     const T       *vin;
     T             *vout;
     const mdp_rtile *tiles;
-    const T       *H;       // [n_spec][M1][16][L/16]: spectrum / M in the order of the row kernel's registers
-    const V2      *tw1;     // [R][256]: W_L^(q (k + a)) when M1 = 1, W_L^(q k) otherwise
+    const T       *H;       // [n_spec][M1][L]: spectrum / M in the order of the row kernel's registers (see h_at)
+    const V2      *tw1;     // [R][256]: W_L^(q (k + a)) when M1 = 1, W_L^(q k) otherwise (see tw_at)
+    const V2      *tw1b;    // the same for the pass back: [R][16][16], q = 16 i + c
     const V2      *tw2;     // [16][16]: W_256^(c k)
     const V2      *wa, *wb; // M1 > 1: W_M^(j2 (k1 + a)) = wa[k1][j2 >> 6] wb[k1][j2 & 63]
     const double  *means;   // [ncols][nb]
@@ -123,16 +124,6 @@ __device__ __forceinline__ bool tile_of(const RArgs<T> &a, int64_t item, Tile<T>
     return true;
 }
 
-__device__ __forceinline__ float ld_stream(const float *p) {  // constant, read once: not kept in L1
-    float v;
-    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_stream(const double *p) {
-    double v;
-    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
 __device__ __forceinline__ float ld_sample(const float *p) {  // from the kernel before (as ld_after), read once
     float v;
     asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
@@ -217,8 +208,13 @@ __device__ __forceinline__ CP<mono64> get_l2(const REnt<mono64> *p) {
     return {Pr<mono64>{v.x}, Pr<mono64>{v.y}};
 }
 
-// CTAs of 256 threads an SM: four FP32 ones (64 registers a thread: 16 points take 32), two FP64 ones
-template <typename T> constexpr int rt_ctas() { return sizeof(T) == 4 ? 4 : 2; }
+// CTAs of 256 threads an SM that transform rows: three FP32 ones (80 registers a thread: 16 points
+// take 32, the 16-byte loads of twiddles and spectrum in flight the rest), two FP64 ones.  Columns: four.
+// 64 x 2^20 samples, half bandwidth 2^14: 4-byte spectrum and 8-byte twiddle loads 623 us at four CTAs
+// (64 registers), 641 at three; 16-byte loads 632 at four, 588 at three; with four for the columns 583.
+// FP64 spectrum loads of 16 bytes: 1224 -> 1190 us.
+template <typename T> constexpr int rt_ctas() { return sizeof(T) == 4 ? 3 : 2; }
+template <typename T> constexpr int rt_col_ctas() { return sizeof(T) == 4 ? 4 : 2; }
 
 // ------------------------------------------------------------------ rows
 // Row of L = R 256 points, L/16 threads, 16 points a thread in every pass.
@@ -228,12 +224,56 @@ template <typename T> constexpr int rt_ctas() { return sizeof(T) == 4 ? 4 : 2; }
 // then the product and the same passes from the other end.  Bound: the FP and
 // shared-memory pipes (4 exchanges of 32 bytes an entry).
 
+// Tables are read 16 bytes at a time: FP32 twiddles of two consecutive k lie side by side ([k/2][n][2]
+// instead of [k][n]), a thread's spectrum values four (FP32) or two (FP64) together.
+template <typename V2> __host__ __device__ constexpr int tw_at(int k, int q, int n) {
+    return sizeof(V2) == 8 ? ((k >> 1) * n + q) * 2 + (k & 1) : k * n + q;
+}
+__device__ __forceinline__ void tw_load(const float2 *t, int k, int q, int n, float2 (&w)[2]) {  // k even
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(t) + ((k >> 1) * n + q));
+    w[0] = make_float2(v.x, v.y);
+    w[1] = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void tw_load(const double2 *t, int k, int q, int n, double2 (&w)[1]) { w[0] = __ldg(t + k * n + q); }
+// the registers of a butterfly times their twiddles; FIRST: register 0 has one too
+template <bool FIRST, typename G, int R, typename V2, typename Put>
+__device__ __forceinline__ void twiddled(const CP<G> (&v)[R], const V2 *t, int q, int n, Put put) {
+    constexpr int W = 16 / (int) sizeof(V2);
+#pragma unroll
+    for (int k = 0; k < R; k += W) {
+        V2 w[W];
+        tw_load(t, k, q, n, w);
+#pragma unroll
+        for (int i = 0; i < W; i++) {
+            CP<G> e = v[rev_bits_c(k + i, ilog2_c(R))];
+            if (FIRST || k + i > 0) e = tmul(e, w[i]);
+            put(k + i, REnt<G>{e.x, e.y});
+        }
+    }
+}
+// register k of thread t, nt threads
+template <typename T> __host__ __device__ constexpr int h_at(int k, int t, int nt) {
+    constexpr int W = 16 / (int) sizeof(T);
+    return ((k / W) * nt + t) * W + k % W;
+}
+__device__ __forceinline__ float4 ld_stream4(const float *p) {  // constant, read once: not kept in L1
+    float4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double2 ld_stream4(const double *p) {
+    double2 v;
+    asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
 // passes 1 to 3 of a row: in(n) gives point n; u[rev(k)] = bin of register k.  ONE: quarter shift
 template <typename T, int R, bool ONE, typename In>
 __device__ __forceinline__ void row_forward(REnt<typename LaneOf<T>::Tag> *s, const typename LaneOf<T>::V2 *tw1,
                                             const typename LaneOf<T>::V2 *tw2, In in,
                                             CP<typename LaneOf<T>::Tag> (&u)[16]) {
     using G = typename LaneOf<T>::Tag;
+    using V2 = typename LaneOf<T>::V2;
     constexpr int NT = 16 * R, S = 16 / R;
     const int     t = threadIdx.x, c = t & 15, kh = t >> 4;
 #pragma unroll
@@ -244,23 +284,13 @@ __device__ __forceinline__ void row_forward(REnt<typename LaneOf<T>::Tag> *s, co
         for (int i = 0; i < R; i++) v[i] = in(256 * i + q);
         if constexpr (ONE) quarter_shift<G, R>(v);
         dif_reg<G, R>(v);
-#pragma unroll
-        for (int k = 0; k < R; k++) {
-            CP<G> w = v[rev_bits_c(k, ilog2_c(R))];
-            if (ONE || k > 0) w = tmul(w, __ldg(tw1 + k * 256 + q));
-            s[rt_pos(k * 256 + q)] = REnt<G>{w.x, w.y};
-        }
+        twiddled<ONE>(v, tw1, q, 256, [&](int k, REnt<G> e) { s[rt_pos(k * 256 + q)] = e; });
     }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 16; i++) u[i] = get(s + rt_pos(kh * 256 + 16 * i + c));
     dif_reg<G, 16>(u);
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        CP<G> w = u[rev_bits_c(k, 4)];
-        if (k > 0) w = tmul(w, __ldg(tw2 + k * 16 + c));
-        s[rt_pos(kh * 256 + 16 * k + c)] = REnt<G>{w.x, w.y};
-    }
+    twiddled<false>(u, tw2, c, 16, [&](int k, REnt<G> e) { s[rt_pos(kh * 256 + 16 * k + c)] = e; });
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 16; i++) u[i] = get(s + rt_pos(kh * 256 + 16 * c + i));  // (k_a, k_b) = (kh, c)
@@ -269,28 +299,20 @@ __device__ __forceinline__ void row_forward(REnt<typename LaneOf<T>::Tag> *s, co
 
 // the passes back from z[k] (register k, parts exchanged); out(n, v) takes point n
 template <typename T, int R, bool ONE, typename Out>
-__device__ __forceinline__ void row_back(REnt<typename LaneOf<T>::Tag> *s, const typename LaneOf<T>::V2 *tw1,
+__device__ __forceinline__ void row_back(REnt<typename LaneOf<T>::Tag> *s, const typename LaneOf<T>::V2 *tw1b,
                                          const typename LaneOf<T>::V2 *tw2, CP<typename LaneOf<T>::Tag> (&z)[16],
                                          Out out) {
     using G = typename LaneOf<T>::Tag;
+    using V2 = typename LaneOf<T>::V2;
     constexpr int NT = 16 * R, S = 16 / R;
     const int     t = threadIdx.x, c = t & 15, kh = t >> 4;
     dif_reg<G, 16>(z);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        CP<G> w = z[rev_bits_c(i, 4)];
-        if (i > 0) w = tmul(w, __ldg(tw2 + i * 16 + c));  // W_256^(c k_b), symmetric
-        s[rt_pos(kh * 256 + 16 * c + i)] = REnt<G>{w.x, w.y};
-    }
+    twiddled<false>(z, tw2, c, 16, [&](int i, REnt<G> e) { s[rt_pos(kh * 256 + 16 * c + i)] = e; });  // W_256^(c k_b)
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 16; k++) z[k] = get(s + rt_pos(kh * 256 + 16 * k + c));
     dif_reg<G, 16>(z);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const CP<G> w = tmul(z[rev_bits_c(i, 4)], __ldg(tw1 + kh * 256 + 16 * i + c));
-        s[rt_pos(kh * 256 + 16 * i + c)] = REnt<G>{w.x, w.y};
-    }
+    twiddled<true>(z, tw1b + kh * 256, c, 16, [&](int i, REnt<G> e) { s[rt_pos(kh * 256 + 16 * i + c)] = e; });
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < S; j++) {
@@ -307,14 +329,25 @@ __device__ __forceinline__ void row_back(REnt<typename LaneOf<T>::Tag> *s, const
     }
 }
 
-// z[k] = u[rev(k)] H, real and imaginary parts exchanged
+// z[k] = u[rev(k)] H, real and imaginary parts exchanged; h: the thread's values (nt threads)
 template <typename T, typename G>
 __device__ __forceinline__ void row_product(const CP<G> (&u)[16], const T *h, int nt, CP<G> (&z)[16]) {
+    constexpr int W = 16 / (int) sizeof(T);
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const CP<G> w = u[rev_bits_c(k, 4)];
-        const Pr<G> hk{ld_stream(h + k * nt)};
-        z[k] = CP<G>{pmul(w.y, hk), pmul(w.x, hk)};
+    for (int k = 0; k < 16; k += W) {
+        const auto v = ld_stream4(h + (k / W) * nt * W);
+        T          hk[W];
+        hk[0] = v.x;
+        hk[1] = v.y;
+        if constexpr (W == 4) {
+            hk[2] = v.z;
+            hk[3] = v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < W; i++) {
+            const CP<G> w = u[rev_bits_c(k + i, 4)];
+            z[k + i] = CP<G>{pmul(w.y, Pr<G>{hk[i]}), pmul(w.x, Pr<G>{hk[i]})};
+        }
     }
 }
 
@@ -331,8 +364,8 @@ __global__ void __launch_bounds__(16 * R, rt_ctas<T>() * 16 / R) rt_one_kernel(R
     CP<G>     u[16], z[16];
     const int halo = a.lambda - 1;
     row_forward<T, R, true>(s, a.tw1, a.tw2, [&](int n) { return point(sample(tl, n), sample(tl, n + M)); }, u);
-    row_product(u, a.H + (int64_t) spec * M + threadIdx.x, NT, z);
-    row_back<T, R, true>(s, a.tw1, a.tw2, z, [&](int n, CP<G> y) {
+    row_product(u, a.H + (int64_t) spec * M + threadIdx.x * (16 / sizeof(T)), NT, z);
+    row_back<T, R, true>(s, a.tw1b, a.tw2, z, [&](int n, CP<G> y) {
         put(tl, halo, n, y.y.v);
         put(tl, halo, n + M, y.x.v);
     });
@@ -352,13 +385,13 @@ __global__ void __launch_bounds__(16 * R, R == 16 ? 2 : 32 / R) rt_spec_rows_ker
         if constexpr (ONE) return point(sample(rs, n), sample(rs, n + M));
         else return get(Y + n);
     }, u);
-    const int64_t at = ((a.item0 << a.log_m1) + blockIdx.x) * L + threadIdx.x;
+    const int64_t at = ((a.item0 << a.log_m1) + blockIdx.x) * L;
     const double  sc = 1.0 / (double) M;
 #pragma unroll
     for (int k = 0; k < 16; k++) {
         const double h = u[rev_bits_c(k, 4)].x.v * sc;
-        if (a.H32) a.H32[at + k * NT] = (float) h;
-        else a.H64[at + k * NT] = h;
+        if (a.H32) a.H32[at + h_at<float>(k, threadIdx.x, NT)] = (float) h;
+        else a.H64[at + h_at<double>(k, threadIdx.x, NT)] = h;
     }
 }
 
@@ -430,7 +463,7 @@ __global__ void __launch_bounds__(256, 2) rt_spec_cols_kernel(RArgs<double> a) {
 }
 
 template <typename T, int M1>
-__global__ void __launch_bounds__(256, rt_ctas<T>()) rt_cols_kernel(RArgs<T> a) {
+__global__ void __launch_bounds__(256, rt_col_ctas<T>()) rt_cols_kernel(RArgs<T> a) {
     constexpr int M = M1 * 4096;
     const int     li = blockIdx.x / (unsigned) M1, part = blockIdx.x % (unsigned) M1;
     Tile<T>       tl;
@@ -443,7 +476,7 @@ __global__ void __launch_bounds__(256, rt_ctas<T>()) rt_cols_kernel(RArgs<T> a) 
         cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample(tl, j0 + n), sample(tl, j0 + n + M)); });
 }
 template <typename T, int M1>
-__global__ void __launch_bounds__(256, rt_ctas<T>()) rt_cols_back_kernel(RArgs<T> a) {
+__global__ void __launch_bounds__(256, rt_col_ctas<T>()) rt_cols_back_kernel(RArgs<T> a) {
     constexpr int M = M1 * 4096;
     const int     li = blockIdx.x / (unsigned) M1, part = blockIdx.x % (unsigned) M1;
     Tile<T>       tl;
@@ -464,8 +497,8 @@ __global__ void __launch_bounds__(256, rt_ctas<T>()) rt_rows_kernel(RArgs<T> a) 
     REnt<G> *row = a.Y + (int64_t) blockIdx.x * L;
     CP<G>    u[16], z[16];
     row_forward<T, 16, false>(s, a.tw1, a.tw2, [&](int n) { return get_l2(row + n); }, u);
-    row_product(u, a.H + (((int64_t) spec << a.log_m1) + part) * L + threadIdx.x, 256, z);
-    row_back<T, 16, false>(s, a.tw1, a.tw2, z, [&](int n, CP<G> y) { row[n] = REnt<G>{y.x, y.y}; });
+    row_product(u, a.H + (((int64_t) spec << a.log_m1) + part) * L + threadIdx.x * (16 / sizeof(T)), 256, z);
+    row_back<T, 16, false>(s, a.tw1b, a.tw2, z, [&](int n, CP<G> y) { row[n] = REnt<G>{y.x, y.y}; });
 }
 
 // ------------------------------------------------------------------ host side
@@ -532,37 +565,41 @@ const void *spec_cols_fn(int m1) {
 inline void set2(float2 &o, double x, double y) { o = make_float2((float) x, (float) y); }
 inline void set2(double2 &o, double x, double y) { o = make_double2(x, y); }
 
-// tables of the transform in the order tw1, tw2, wa, wb, one buffer
+// tables of the transform in the order tw1, tw1b, tw2, wa, wb, one buffer
 template <typename V2>
-int build_tables(int m1, int L, DevBuf &buf, const V2 **tw1, const V2 **tw2, const V2 **wa, const V2 **wb) {
+int build_tables(int m1, int L, DevBuf &buf, const V2 **tw1, const V2 **tw1b, const V2 **tw2, const V2 **wa,
+                 const V2 **wb) {
     const int       R = L / 256, M = m1 * L;
-    std::vector<V2> t(L + 256 + (m1 > 1 ? 128 * m1 : 0));
+    const int       B = sizeof(V2) == 8 ? L : 0;  // where tw1b starts: FP64 has one layout for both
+    std::vector<V2> t(B + L + 256 + (m1 > 1 ? 128 * m1 : 0));
     double          re, im;
     for (int k = 0; k < R; k++)
         for (int q = 0; q < 256; q++) {
             // W_L^(q (k - 1/4)) = W_4L^(q (4k - 1)), exponents modulo 4L
             const int64_t e = m1 == 1 ? (int64_t) q * (4 * k - 1) : (int64_t) 4 * q * k;
             mdp_host_cexp((long double) ((e + 4LL * L) % (4LL * L)), 4.0L * L, &re, &im);
-            set2(t[k * 256 + q], re, im);
+            set2(t[tw_at<V2>(k, q, 256)], re, im);
+            set2(t[B + k * 256 + tw_at<V2>(q >> 4, q & 15, 16)], re, im);
         }
     for (int k = 0; k < 16; k++)
         for (int c = 0; c < 16; c++) {
             mdp_host_cexp(k * c, 256, &re, &im);
-            set2(t[L + 16 * k + c], re, im);
+            set2(t[B + L + tw_at<V2>(k, c, 16)], re, im);
         }
     if (m1 > 1)
         for (int k = 0; k < m1; k++)
             for (int h = 0; h < 64; h++) {
                 const int64_t den = 4LL * M, ea = 64LL * h * (4 * k - 1), eb = (int64_t) h * (4 * k - 1);
                 mdp_host_cexp((long double) ((ea + den) % den), (long double) den, &re, &im);
-                set2(t[L + 256 + 64 * k + h], re, im);
+                set2(t[B + L + 256 + 64 * k + h], re, im);
                 mdp_host_cexp((long double) ((eb + den) % den), (long double) den, &re, &im);
-                set2(t[L + 256 + 64 * m1 + 64 * k + h], re, im);
+                set2(t[B + L + 256 + 64 * m1 + 64 * k + h], re, im);
             }
     MDP_TRY(buf.alloc(sizeof(V2) * t.size()));
     MDP_CUDA(cudaMemcpy(buf.p, t.data(), sizeof(V2) * t.size(), cudaMemcpyHostToDevice));
     *tw1 = buf.as<V2>();
-    *tw2 = *tw1 + L;
+    *tw1b = *tw1 + B;
+    *tw2 = *tw1b + L;
     *wa = *tw2 + 256;
     *wb = *wa + 64 * m1;
     return MDP_OK;
@@ -595,8 +632,8 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
         if (!tiles.empty())
             MDP_CUDA(cudaMemcpy(P.tile_start.p, tiles.data(), sizeof(mdp_rtile) * tiles.size(), cudaMemcpyHostToDevice));
     }
-    const V2 *p[4];
-    MDP_TRY(build_tables<V2>(m1, L, P.ltw, &p[0], &p[1], &p[2], &p[3]));
+    const V2 *p[5];
+    MDP_TRY(build_tables<V2>(m1, L, P.ltw, &p[0], &p[1], &p[2], &p[3], &p[4]));
     if (m1 > 1) {
         // FP32 plans also run column batches of up to 8 columns
         const int64_t items = std::max<int64_t>(1, P.n_tiles * (sizeof(T) == 4 ? 8 : 1));
@@ -614,7 +651,7 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
     }
     RArgs<double> a{};
     DevBuf        tab, rows, Y;
-    MDP_TRY(build_tables<double2>(m1, L, tab, &a.tw1, &a.tw2, &a.wa, &a.wb));
+    MDP_TRY(build_tables<double2>(m1, L, tab, &a.tw1, &a.tw1b, &a.tw2, &a.wa, &a.wb));
     MDP_TRY(rows.alloc(sizeof(double) * N->h_Tuniq.size()));
     MDP_CUDA(cudaMemcpyAsync(rows.p, N->h_Tuniq.data(), sizeof(double) * N->h_Tuniq.size(), cudaMemcpyHostToDevice,
                              ctx->stream));
@@ -654,7 +691,8 @@ int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, c
     a.tiles = P.tile_start.as<mdp_rtile>();
     a.H = P.spectra.as<T>();
     a.tw1 = P.ltw.as<V2>();
-    a.tw2 = a.tw1 + L;
+    a.tw1b = a.tw1 + (sizeof(V2) == 8 ? L : 0);
+    a.tw2 = a.tw1b + L;
     a.wa = a.tw2 + 256;
     a.wb = a.wa + 64 * m1;
     a.means = d_means;
