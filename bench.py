@@ -210,6 +210,11 @@ def ninv_kernel(t: dict, prec: str) -> str:
     if t.get("cluster_four_step"):
         m1, m2 = t["cluster_four_step"]
         return f"ninv4_kernel<{prec}, {t['cluster']}> ({m1}x{m2} cluster four-step tiles)"
+    if t.get("right_angle"):
+        m1, m2 = t["right_angle"]
+        if m1 == 1:
+            return f"rt_one_kernel<{prec}, {m2 // 256}> (right-angle tiles of {m2} points)"
+        return f"rt_cols_kernel + rt_rows_kernel + rt_cols_back_kernel<{prec}> ({m1}x{m2} right-angle tiles)"
     if t.get("split"):
         m1, m2 = t["split"]
         return f"split_cols_kernel + split_rows_kernel + split_cols_kernel<{prec}> ({m1}x{m2} four-step tiles)"
@@ -869,7 +874,10 @@ def main():
                 "traffic": traffic, "peak_source": "measured" if peaks else "fallback",
                 "per_application_ms": {k: round(v, 4) for k, v in per.items()},
                 "algorithmic_bytes": ab}
-    if dom == "Ninv" and ninv_tile.get("split"):
+    if dom == "Ninv" and ninv_tile.get("right_angle"):
+        roofline["limiter"] = ("not DRAM (the scratch of a group of tiles stays in L2): in FP32 the row kernel's "
+                               "shared memory and instruction issue, in FP64 its load latency at 16 warps an SM (ncu)")
+    elif dom == "Ninv" and ninv_tile.get("split"):
         # what the ncu captures show about the split kernels
         roofline["limiter"] = ("not DRAM (1.8-2.7 TB/s of DRAM traffic, ~3x the algorithmic bytes from the "
                                "four-step scratch): instruction issue in the row and inverse-column passes (issue "

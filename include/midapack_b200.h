@@ -114,7 +114,10 @@ int  mdp_prepare_fp32(mdp_context *ctx, mdp_pointing *A, mdp_noise *N);
  * (three kernels, four-step FFT of 2^split_log_m1 x 2^split_log_m2 points)
  * reports split_log_m1 > 0 and cluster 0; a cluster four-step plan (one
  * cluster of C CTAs per tile, 2C x 4096 points, the tile on chip) reports
- * split_log_m1 = log2(2C), split_log_m2 = 12 and cluster C.  The autotuner runs
+ * split_log_m1 = log2(2C), split_log_m2 = 12 and cluster C; a right-angle plan
+ * of M1 x 4096 points reports split_log_m1 = log2(M1) > 0, split_log_m2 = 12 and
+ * cluster 0, one of a single row split_log_m1 = 0 and split_log_m2 = log2 of its
+ * points (0 for the other one-kernel plans).  The autotuner runs
  * once per precision, band (ceil log2 lambda) and block length class. */
 int  mdp_noise_plan(mdp_context *ctx, mdp_noise *N, int fp32, int *log2_cta_points, int *cluster_ctas,
                     int *threads, int *tuned, int *split_log_m1, int *split_log_m2);

@@ -309,7 +309,7 @@ class Noise:
 
     def set_plan(self, plan: str, fp32: bool = False):
         """Replaces the tile plan of one precision (see mdp_noise_set_plan):
-        "auto", "model", "fft:N", "log2_ml,cluster,threads", "s,log_m1,log_m2", "c,C"."""
+        "auto", "model", "fft:N", "log2_ml,cluster,threads", "s,log_m1,log_m2", "c,C", "r,log_m1,log_m2"."""
         check(lib().mdp_noise_set_plan(self.ctx.h, self.h, int(fp32), plan.encode()), "mdp_noise_set_plan")
         return self
 
@@ -319,9 +319,12 @@ class Noise:
                                    ct.byref(s1), ct.byref(s2)))
         if s1.value and c.value:
             return dict(cluster_four_step=[1 << s1.value, 1 << s2.value], tuned=bool(tu.value))
+        out = dict(tuned=bool(tu.value))
+        if s2.value >= (12 if s1.value else 1):  # right-angle tiles: rows of 4096 points, or one row
+            out["right_angle"] = [1 << s1.value, 1 << s2.value]
         if s1.value:
-            return dict(split=[1 << s1.value, 1 << s2.value], tuned=bool(tu.value))
-        return dict(cta_points=1 << lm.value, threads=th.value, tuned=bool(tu.value))
+            return dict(out, split=[1 << s1.value, 1 << s2.value])
+        return dict(out, cta_points=1 << lm.value, threads=th.value)
 
     def tile(self):
         n, c, t = ct.c_int(), ct.c_int(), ct.c_int64()

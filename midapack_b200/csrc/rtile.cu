@@ -36,8 +36,8 @@
 //
 // Measured against the best of the even/odd-packed plans on a B200 (64 x 2^20 samples,
 // half bandwidth 2^14): FP32 0.93 -> 0.58 ms, error against 64 bits 5.9e-7 -> 2.7e-7; FP64
-// 1.62 -> 1.19 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 76 % busy in
-// FP32, waiting for its loads in FP64.  A spectrum from the transform itself takes
+// 1.62 -> 1.19 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 74 % busy in
+// FP32, waiting for its loads in FP64; the columns wait for theirs.  A spectrum from the transform itself takes
 // microseconds where the direct cosine sums took 3.7 ms (half bandwidth 2^13, 2^17 samples).
 #include <algorithm>
 #include <cmath>
@@ -221,8 +221,9 @@ template <typename T> constexpr int rt_col_ctas() { return sizeof(T) == 4 ? 4 : 
 //   pass 1  n = 256 a + q over a (R points; 16/R columns q a thread), times tw1
 //   pass 2  q = 16 b + c over b, thread (k_a, c), times tw2
 //   pass 3  over c, thread (k_a, k_b): bins k_a + R (k_b + 16 k_c), k_c = register
-// then the product and the same passes from the other end.  Bound: the FP and
-// shared-memory pipes (4 exchanges of 32 bytes an entry).
+// then the product and the same passes from the other end.  Bound: FP32 shared memory
+// and issue (four exchanges of a write and a read of each 8-byte point: L1 74 % busy, 48 % of
+// the issue slots), FP64 (16-byte points: 62 %, 25 %) the latency of its loads at 16 warps an SM.
 
 // Tables are read 16 bytes at a time: FP32 twiddles of two consecutive k lie side by side ([k/2][n][2]
 // instead of [k][n]), a thread's spectrum values four (FP32) or two (FP64) together.

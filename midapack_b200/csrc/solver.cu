@@ -1232,7 +1232,6 @@ extern "C" int mdp_local_blocks(mdp_context *ctx, mdp_pointing *A, const mdp_noi
     }
     MDP_CUDA(cudaSetDevice(ctx->device));
     const int64_t npix = A->n_map() / 3;
-    cudaStream_t  st = ctx->stream;
     MDP_TRY(localW_launch(ctx, A, N, d_W, d_hits));
     return MDP_OK;
 }

@@ -8,8 +8,11 @@
 // tile stride bs - 2(lambda-1), zero padding outside the block),
 // 569-616 (scmm_direct: forward FFT, spectrum product, inverse FFT).
 //
-// B200 design.  All tiles of all blocks run in one launch: one CTA (or one
-// thread-block cluster of C CTAs sharing the FFT through distributed shared
+// B200 design.  The automatic choice is among right-angle tiles (rtile.cu) and
+// the shortest of the one-kernel tiles of this file; the longer ones, the split
+// tiles (three kernels) and the cluster four-step tiles (ninv4.cu) are plans by
+// name.  One-kernel tiles: all tiles of all blocks run in one launch, one CTA (or
+// one thread-block cluster of C CTAs sharing the FFT through distributed shared
 // memory) per overlap-save tile.  A tile of N real samples is packed as N/2
 // complex points z[j] = x[2j] + i x[2j+1]; the complex FFT is an in-place
 // radix-2 decimation-in-frequency transform executed as radix-16 register
@@ -1136,20 +1139,6 @@ static int64_t cand_E(const TileCand &c, int lambda) {
     return cand_N(c) - 2LL * (lambda - 1) - (c.split == 1 || c.split == 2 ? 1 : 0);
 }
 
-// split plans: columns of 16 <= M1 <= 2^m1max points, rows of 32 <= M2 <= 512
-// points; shapes whose transforms end in a lone radix-2 pass (5 or 9 bits) are
-// kept only when no other shape gives the same M
-static std::vector<std::pair<int, int>> split_shapes(int logM, int m1max) {
-    std::vector<std::pair<int, int>> all, good;
-    for (int a = 4; a <= m1max; a++) {
-        const int b = logM - a;
-        if (b < 5 || b > 9) continue;
-        all.push_back({a, b});
-        if (a % 4 != 1 && b % 4 != 1) good.push_back({a, b});
-    }
-    return good.empty() ? all : good;
-}
-
 static int default_threads(int log_ml) { return std::min(512, std::max(64, (1 << log_ml) / 16)); }
 
 static int ceil_log2_i(int64_t v) {
@@ -1163,9 +1152,9 @@ static int ceil_log2_i(int64_t v) {
 // for blocks and bands shorter than the smallest right-angle tile.  The longer
 // one-kernel tiles, the split and the cluster four-step tiles were slower than the
 // best right-angle tile at every size timed (blocks of 500 to 2^23 samples, half
-// bandwidths 20 to 2^14, e.g. 64 x 2^20 samples, 2^14: FP64 1.64 -> 1.45 ms, FP32
-// 0.94 -> 0.71 ms; 8 x 2^23, 8192: 1.48 -> 1.26, 0.82 -> 0.64 ms; at the small end
-// 2000 x 500 samples, 20: 38 -> 25 us); they remain plans by name.
+// bandwidths 20 to 2^14, e.g. 64 x 2^20 samples, 2^14: FP64 1.62 against 1.19 ms, FP32
+// 0.93 against 0.585 ms; 24 blocks of 350001 to 700001, 3001: FP32 220 against 118 us;
+// at the small end 2000 x 500 samples, 20: 38 against 25 us); they remain plans by name.
 template <typename T>
 static std::vector<TileCand> tile_candidates(int lambda) {
     std::vector<TileCand> out;
