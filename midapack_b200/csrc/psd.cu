@@ -72,13 +72,23 @@ __device__ __forceinline__ double2 expi(double turns_pi, double sign) {
     sincospi(turns_pi, &s, &c);
     return make_double2(c, sign * s);
 }
-// exp(sign i pi m^2 / n): m^2 < 2^48 reduced modulo 2n exactly
-__device__ __forceinline__ double2 chirp1(int m, int n, double sign) {
-    const uint64_t mm = (uint64_t) m * (uint64_t) m, n2 = 2 * (uint64_t) n;
-    int64_t        r = (int64_t) (mm - (uint64_t) ((double) mm / (double) n2) * n2);
-    if (r < 0) r += n2;
-    if (r >= (int64_t) n2) r -= n2;
-    return expi((double) r / (double) n, sign);
+// a / n for many a and one n: the quotient by the reciprocal and one step of residual correction
+// (Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990), within an
+// ulp of the correctly rounded one, in place of a division each
+struct Recip {
+    double n, inv;
+    __device__ __forceinline__ double div(double a) const {
+        const double q = a * inv;
+        return fma(fma(-q, n, a), inv, q);
+    }
+};
+// exp(sign i pi m^2 / n): m^2 < 2^48 reduced modulo 2n exactly (whole numbers below 2^53)
+__device__ __forceinline__ double2 chirp1(int m, const Recip &n, double sign) {
+    const double mm = (double) m * (double) m, n2 = 2.0 * n.n;
+    double       r = fma(-trunc(mm * (0.5 * n.inv)), n2, mm);
+    if (r < 0.0) r += n2;
+    if (r >= n2) r -= n2;
+    return expi(n.div(r), sign);
 }
 
 __global__ void psd_tables_kernel(double2 *tw1, double2 *tw2, double2 *tw4k) {
@@ -128,6 +138,7 @@ __global__ void __launch_bounds__(kT) psd_sums_final_kernel(const double *part, 
 struct Load {
     const double *x;
     double        mean, slope, c;
+    Recip         rn;       // of n
     int           n, kind;  // 0: samples, 1: chirped samples, 2: filter
     int           L;
 };
@@ -136,14 +147,14 @@ __device__ __forceinline__ C1 point(const Load &l, int j) {
         // exp(i pi m^2 / n) for -n < m <= n/2, negative m at L + m
         const int m = j <= l.n / 2 ? j : (j > l.L - l.n ? l.L - j : -1);
         if (m < 0) return mk(0.0, 0.0);
-        const double2 w = chirp1(m, l.n, 1.0);
+        const double2 w = chirp1(m, l.rn, 1.0);
         return mk(w.x, w.y);
     }
     if (j >= l.n) return mk(0.0, 0.0);
-    const double w = 0.5 - 0.5 * cospi((double) (2 * j) / (double) l.n);
+    const double w = 0.5 - 0.5 * cospi(l.rn.div((double) (2 * j)));
     const double v = (__ldg(l.x + j) - l.mean - l.slope * ((double) j - l.c)) * w;
     if (l.kind == 0) return mk(v, 0.0);
-    const double2 ch = chirp1(j, l.n, -1.0);
+    const double2 ch = chirp1(j, l.rn, -1.0);
     return mk(v * ch.x, v * ch.y);
 }
 
@@ -181,6 +192,7 @@ __global__ void __launch_bounds__(kT, 2) psd_cols_kernel(PsdArgs a) {
             l.n = a.fn[item - a.cnt];
             l.kind = 2;
         }
+        l.rn = Recip{(double) l.n, 1.0 / (double) l.n};
     }
     auto twl = [&](int k1, int c) {  // W_L^(j2 k1), j2 = c0 + c, j2 k1 < L
         return expi((double) ((c0 + c) * k1) / (2048.0 * N1), -1.0);
