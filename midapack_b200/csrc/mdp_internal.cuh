@@ -256,10 +256,15 @@ struct mdp_chunks {
     double        *partial, *means;
 };
 
+// One arrival of n at *count: true for the last.  The count goes back to zero by itself with it, so it
+// needs no reset and holds for any number of rounds.  (A free-running count taken modulo n does not: it
+// wraps at 2^32, which is a multiple of n only when n is a power of two.)
+__device__ __forceinline__ bool last_arrival(uint32_t *count, uint32_t n) { return atomicInc(count, n - 1u) == n - 1u; }
+
 // The end of a CTA that has summed its chunk blockIdx.x: its partial sum from the threads' acc,
 // and the block's mean by the CTA that finishes the block's last chunk (the partial sums in a
 // fixed order: lane l takes l, l + 32, ..., then the lanes pairwise).  All threads of the CTA, at
-// most 1024.  `arrived` counts modulo the block's chunks, so that it needs no reset; null: the
+// most 1024.  `arrived` counts the block's chunks (last_arrival); null: the
 // partial sum only, the means are a kernel of their own.  That is the rule above MDP_MEAN_CHUNKS
 // chunks (one wave of CTAs): the fence and the count keep a CTA's slot for 1-2 us, which a
 // second wave waits for (P of 8 x 2^20 rows: 5 us more than the 4 us of the other kernel);
@@ -280,14 +285,13 @@ __device__ __forceinline__ void chunk_mean(const mdp_chunks &c, double acc) {
     }
     const int b = c.blk[blockIdx.x], n = c.blk_nchunk[b];
     if (n > 1) {
-        uint32_t prev = 0;
+        bool last = false;
         if (lane == 0) {
             c.partial[blockIdx.x] = v;
             __threadfence();
-            prev = atomicAdd(c.arrived + b, 1u);
+            last = last_arrival(c.arrived + b, (uint32_t) n);
         }
-        prev = __shfl_sync(0xffffffffu, prev, 0);
-        if ((prev + 1u) % (uint32_t) n != 0u) return;
+        if (!__shfl_sync(0xffffffffu, (int) last, 0)) return;
         __threadfence();
         const double *p = c.partial + c.blk_chunk0[b];
         v = 0.0;
@@ -331,7 +335,7 @@ struct mdp_noise {
     DevBuf               blk_chunk0;     // int32 [nb] first chunk of each block
     DevBuf               blk_nchunk;     // int32 [nb]
     DevBuf               chunk_blk;      // int32 [n_chunks] block of each chunk
-    DevBuf               arrived;        // uint32 [nb] chunks of a block finished, modulo its chunks
+    DevBuf               arrived;        // uint32 [nb] chunks of a block finished in this application (zero between)
     DevBuf               partial;        // double [n_chunks] chunk sums
     mdp_chunks           chunks(double *d_partial, double *d_means) const {
         return mdp_chunks{chunk_start.as<int64_t>(), chunk_len.as<int32_t>(), chunk_blk.as<int32_t>(),

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(512) mr_matvec32_kernel(const int32_t *__restr
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        is_last = (atomicAdd(c.arrived + b, 1u) + 1u) % (uint32_t) nc == 0u;
+        is_last = last_arrival(c.arrived + b, (uint32_t) nc);
         __threadfence();
     }
     __syncthreads();
