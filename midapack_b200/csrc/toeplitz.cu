@@ -1149,24 +1149,33 @@ static int ceil_log2_i(int64_t v) {
 
 // The configurations whose tile holds the band (E >= 1) that the automatic choice
 // considers: every right-angle shape, and the one-CTA tiles of up to 2^8 points
-// for blocks and bands shorter than the smallest right-angle tile.  The longer
-// one-kernel tiles, the split and the cluster four-step tiles were slower than the
+// for blocks and bands shorter than the smallest right-angle tile.  The other
+// one-kernel tiles, the shorter split and the cluster four-step tiles were slower than the
 // best right-angle tile at every size timed (blocks of 500 to 2^23 samples, half
 // bandwidths 20 to 2^14, e.g. 64 x 2^20 samples, 2^14: FP64 1.62 against 1.19 ms, FP32
 // 0.93 against 0.585 ms; 24 blocks of 350001 to 700001, 3001: FP32 220 against 118 us;
 // at the small end 2000 x 500 samples, 20: 38 against 25 us); they remain plans by name.
+//
+// Bands that leave the longest right-angle tile (2^17 samples) less than half useful take the
+// split tile of 2^18 samples too, the only kind that holds half bandwidths above 2^16.
+// 8 x 2^20 samples, right-angle 16 x 4096 against split 256 x 512, us: half bandwidth
+// 32768 FP64 219 : 271, FP32 99 : 162; 40000 289 : 272, 125 : 162; 50000 424 : 303, 186 : 178;
+// 65536, where a right-angle tile has two outputs, split 335 and 195.  (Split 512 x 256 was 5 % slower in FP32
+// and the cluster tile of 2^18 samples 40-67 %.)  Less than a quarter useful, FP32 takes that cluster
+// tile: its points stay on chip, where the split tile's scratch grows to many times the samples.
 template <typename T>
 static std::vector<TileCand> tile_candidates(int lambda) {
     std::vector<TileCand> out;
-    for (int lml = 6; lml <= 8; lml++) {
-        TileCand c{lml, 1, default_threads(lml)};
+    auto add = [&](const TileCand &c) {
         if (cand_E(c, lambda) >= 1) out.push_back(c);
-    }
+    };
+    for (int lml = 6; lml <= 8; lml++) add(TileCand{lml, 1, default_threads(lml)});
     for (int a = 0; a <= 4; a++)
-        for (int b = 9; b <= 12; b++) {
-            TileCand c{0, 0, 0, 3, a, b};
-            if (rtile_shape(a, b) && cand_E(c, lambda) >= 1) out.push_back(c);
-        }
+        for (int b = 9; b <= 12; b++)
+            if (rtile_shape(a, b)) add(TileCand{0, 0, 0, 3, a, b});
+    const TileCand longest{0, 0, 0, 3, 4, 12}, wide{0, 0, 0, 1, 8, 9};
+    if (2 * cand_E(longest, lambda) < cand_N(longest))
+        add(sizeof(T) == 4 && 4 * cand_E(wide, lambda) < cand_N(wide) ? TileCand{14, 8, default_threads(14)} : wide);
     return out;
 }
 
@@ -1195,7 +1204,9 @@ static double tile_model_cost(const TileCand &c, int lambda, int64_t max_block) 
     const double  eff = (double) std::min<int64_t>(E, std::max<int64_t>(max_block, 1));
     double        cost = (double) N / eff * (logN + 3);
     if (c.split == 3) {
-        cost *= c.log_m1 ? 0.5 : 0.4;  // no untangle, paired-lane arithmetic; scratch round trips of the columns
+        cost *= c.log_m1 ? 0.5 : 0.4;  // no untangle; scratch round trips of the columns
+    } else if (c.split == 1) {
+        cost *= 0.75;  // 1.4 (FP64) to 1.6 times (FP32) the columns-and-rows right-angle tile's time a sample
     } else {
         if (c.C > 1) cost += 3.0 * std::log2((double) c.C);
         if (c.threads != default_threads(c.log_ml)) cost *= 1.01;  // ties go to the default launch shape
