@@ -1221,19 +1221,26 @@ template <typename T>
 static int launch_tiles(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, const T *d_in, T *d_out,
                         const double *d_means, int ncols = 1, int64_t col_stride = 0, const int *d_active = nullptr);
 
-// Autotuner.  The plans of a precision are keyed by the band (ceil log2 of
-// lambda), the block length (ceil log2) and the rows (ceil log2, at most 2^24: a few
-// tiles leave most of the device idle, where shorter tiles win); the first noise operator with a
-// new key times every candidate kept by the screen below on a sample of its
+// Autotuner.  The plans of a precision are keyed by the candidates that pass the screen below and which
+// of them are a quarter useful, the band (ceil log2 of lambda), the block length (ceil log2) and the rows
+// (ceil log2, at most 2^24: a few tiles leave most of the device idle, where shorter tiles win); the first
+// noise operator with a new key times every one of them on a sample of its
 // own blocks (at most 2^24 rows, zero data: the tile kernels do the same work
-// whatever the values) and the fastest per useful row is kept for the process.
+// whatever the values) and the fastest per useful row is kept for the process.  (Without the
+// candidates in the key the tile of 2048 samples that won at half bandwidth 513 was taken for all to 1024,
+// where two of its samples are outputs: 4 x 12000 samples, FP64 14.4 -> 197 us, FP32 9.9 -> 98.8 us.)
 struct TuneKey {
-    int prec, lam_bits, blk_bits, row_bits, device;
+    int      prec, lam_bits, blk_bits, row_bits, device;
+    uint64_t screen;  // cand_bit of each, and 32 bits up of those a quarter useful
     bool operator<(const TuneKey &o) const {
-        return std::tie(prec, lam_bits, blk_bits, row_bits, device) <
-               std::tie(o.prec, o.lam_bits, o.blk_bits, o.row_bits, o.device);
+        return std::tie(prec, lam_bits, blk_bits, row_bits, device, screen) <
+               std::tie(o.prec, o.lam_bits, o.blk_bits, o.row_bits, o.device, o.screen);
     }
 };
+// a bit of its own for every candidate of the automatic choice
+static uint64_t cand_bit(const TileCand &c) {
+    return uint64_t(1) << (c.split == 3 ? (c.log_m1 ? 3 + c.log_m1 : c.log_m2 - 9) : c.split ? 8 : 3 + c.log_ml);
+}
 static std::mutex                   g_tune_mu;
 static std::map<TuneKey, TileCand> g_tuned;
 
@@ -1358,24 +1365,25 @@ static int choose_plan(mdp_context *ctx, const mdp_noise *N, TileCand *out, int 
     });
     *out = cands[0];
     if (forced || !tune || cands.size() == 1) return MDP_OK;
-    // screen: tiles at least a quarter useful and not longer than twice the block plus the halo
+    // screen: tiles at least an eighth useful and not longer than twice the block plus the halo (a quarter left
+    // out the tile of 2048 samples at half bandwidth 900, the faster one for 4 x 12000: 12.7 against 14.9 us)
     std::vector<TileCand> screen;
+    uint64_t              bits = 0;
     for (const TileCand &c : cands) {
         const int64_t Nn = cand_N(c), E = cand_E(c, N->lambda);
-        if (E * 4 >= Nn && E <= 2 * std::max<int64_t>(N->max_block, 1) + 2LL * N->lambda) screen.push_back(c);
+        if (E * 8 < Nn || E > 2 * std::max<int64_t>(N->max_block, 1) + 2LL * N->lambda) continue;
+        screen.push_back(c);
+        bits |= cand_bit(c) | (E * 4 < Nn ? 0 : cand_bit(c) << 32);
     }
     if (screen.size() <= 1) return MDP_OK;
     const TuneKey key{f32 ? 32 : 64, ceil_log2(N->lambda), ceil_log2(std::max<int64_t>(N->max_block, 1)),
-                      std::min(24, ceil_log2(std::max<int64_t>(N->nrow_end, 1))), ctx->device};
+                      std::min(24, ceil_log2(std::max<int64_t>(N->nrow_end, 1))), ctx->device, bits};
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto                        it = g_tuned.find(key);
     if (it != g_tuned.end()) {
-        const TileCand &c = it->second;
-        if (cand_E(c, N->lambda) >= 1) {
-            *out = c;
-            *tuned = 1;
-            return MDP_OK;
-        }
+        *out = it->second;
+        *tuned = 1;
+        return MDP_OK;
     }
     TileCand best = screen[0];
     MDP_TRY(tune_plan<T>(ctx, N, screen, &best));
