@@ -226,7 +226,8 @@ struct mdp_tile_plan {
                            // 2: cluster four-step (ninv4.cu: C = cluster CTAs, M = 2C x 4096 points);
                            // 3: right-angle tiles (rtile.cu, M = 2^log_m1 x 2^log_m2 points)
     int     log_m1 = 0, log_m2 = 0;  // split: M = 2^log_m1 * 2^log_m2 complex points per tile
-    DevBuf  scratch;       // split: [n_tiles][M] complex work array; right-angle tiles: two launch groups'
+    DevBuf  scratch;       // split: [n_tiles][M] complex work array; right-angle tiles: [scratch_items][M]
+    int64_t scratch_items = 0;  // right-angle tiles: at most two launch groups'
     DevBuf  ltw2, wa, wb;  // split: row-pass twiddles, W_M factor tables
     int     log2_ml = 0;   // per-CTA complex points = 2^log2_ml
     int     cluster = 1;   // CTAs per tile

@@ -510,16 +510,20 @@ template <typename T> size_t rows_smem(int L) { return 2 * sizeof(T) * (size_t) 
 // and the next launch share the device with the other group's.  64 x 2^20 samples, half
 // bandwidth 2^14, one stream and 64 MB -> two and 64 MB each: FP32 0.70 -> 0.645 ms, FP64 1.34
 // -> 1.20 ms (halves of 24, 32, 48 MB: 0.68, 0.66, 0.64 and 1.24, 1.21, 1.24 ms); work that fits
-// one half is cut in two from 2 x 16 MB on (8 x 2^20, 2^13, FP32: 99 -> 96 us).
+// one half is cut in two from 2 x 16 MB on (8 x 2^20, 2^13, FP32: 99 -> 96 us), and less is one group (2^20
+// samples, half bandwidth 2^13, FP64: 41.0 us in two groups, 34.4 in one; FP32, 18 MB in all: 42.3 and 37.6 us).
 constexpr int64_t RT_HALF_BYTES = int64_t(64) << 20, RT_MIN_BYTES = int64_t(16) << 20;
 struct Groups {
     int64_t n, per;  // how many, items in each but the last
 };
+constexpr int64_t half_items(int64_t item_bytes) { return std::max<int64_t>(1, RT_HALF_BYTES / item_bytes); }
+// of `items` items with scratch for `cap` of them: all at once, in two halves, or (cap < items) in
+// groups of half the scratch; n = 1 is one group on the context's stream
 Groups groups_of(int64_t items, int64_t item_bytes, int64_t cap) {
-    const int64_t half = std::min<int64_t>(RT_HALF_BYTES, cap / 2 >= item_bytes ? cap / 2 : cap);
-    int64_t       n = std::max<int64_t>(1, (items * item_bytes + half - 1) / half);
+    const int64_t half = std::min(half_items(item_bytes), items <= cap ? items : std::max<int64_t>(1, cap / 2));
+    int64_t       n = (items + half - 1) / half;
     if (n == 1 && items > 1 && items * item_bytes >= 2 * RT_MIN_BYTES) n = 2;
-    const int64_t per = std::min<int64_t>((items + n - 1) / n, std::max<int64_t>(1, half / item_bytes));
+    const int64_t per = (items + n - 1) / n;
     return Groups{(items + per - 1) / per, per};
 }
 
@@ -637,9 +641,10 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
     MDP_TRY(build_tables<V2>(m1, L, P.ltw, &p[0], &p[1], &p[2], &p[3], &p[4]));
     if (m1 > 1) {
         // FP32 plans also run column batches of up to 8 columns
+        const int64_t item_bytes = 2 * (int64_t) sizeof(T) * M;
         const int64_t items = std::max<int64_t>(1, P.n_tiles * (sizeof(T) == 4 ? 8 : 1));
-        const int64_t most = std::max<int64_t>(2, 2 * RT_HALF_BYTES / (int64_t) (2 * sizeof(T) * M));
-        MDP_TRY(P.scratch.alloc(2 * sizeof(T) * (size_t) M * (size_t) std::min(items, most)));
+        P.scratch_items = std::max<int64_t>(2, std::min(items, 2 * half_items(item_bytes)));
+        MDP_TRY(P.scratch.alloc((size_t) (P.scratch_items * item_bytes)));
         MDP_CUDA(cudaFuncSetAttribute((const void *) rt_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<T>(L)));
     } else {
         MDP_CUDA(cudaFuncSetAttribute(one_fn<T>(L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rows_smem<T>(L)));
@@ -720,7 +725,7 @@ int rtile_launch(mdp_context *ctx, const mdp_noise *N, const mdp_tile_plan &P, c
         return MDP_OK;
     };
     if (m1 == 1) return launch(one_fn<T>(L), dim3((unsigned) items), L / 16, rows_smem<T>(L), ctx->stream, true);
-    const Groups g = groups_of(items, 2 * (int64_t) sizeof(T) * M, (int64_t) P.scratch.bytes);
+    const Groups g = groups_of(items, 2 * (int64_t) sizeof(T) * M, P.scratch_items);
     cudaStream_t st[2] = {ctx->stream, ctx->stream};
     if (g.n > 1) {
         MDP_TRY(mdp_side_fork(ctx));
