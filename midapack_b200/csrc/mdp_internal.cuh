@@ -102,6 +102,14 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 int  mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev);
 void mdp_mem_put(void *p, size_t bytes, int dev);
 void mdp_mem_trim(int dev);  // gives the device's cached blocks back to the driver
+// what a thread releases inside it enters the cache at its end, after one wait (for destroying
+// objects of many buffers, not for code that allocates)
+struct mdp_mem_scope {
+    mdp_mem_scope();
+    ~mdp_mem_scope();
+    mdp_mem_scope(const mdp_mem_scope &) = delete;
+    mdp_mem_scope &operator=(const mdp_mem_scope &) = delete;
+};
 
 struct DevBuf {
     void  *p     = nullptr;

@@ -6,9 +6,11 @@
 // (MatLocalShape), 704-729 (MatVecProd), 819-859 (TrMatVecProd);
 // algebra/src/mapmat/csort.c:111-135 (counting_sort), cindex.c:34-42,102-116
 // (sindex/dichotomy).
+#include <algorithm>
 #include <cstdarg>
 #include <cstring>
 #include <deque>
+#include <map>
 #include <mutex>
 
 #include "mdp_internal.cuh"
@@ -45,6 +47,12 @@ extern "C" const char *mdp_strerror(int code) {
 // driver, all of a device's on mdp_context_trim or when the driver is out of memory.
 // Sizes are rounded up so that blocks fit again; a block is taken for a request of at
 // least three quarters of it.
+//
+// A block enters the cache after a wait for all that is queued on its device, which is also what
+// a caller that frees its own arrays after closing an object relies on.  The wait is a cudaFree,
+// of 512 bytes beside 512 that stay allocated (2 us to allocate, 3 us to free on an idle
+// device; alone, with a segment to map, 0.6 ms): cudaFree is allowed while another thread
+// captures a stream in thread-local mode, where cudaDeviceSynchronize (3 us) ends that capture.
 namespace {
 constexpr size_t kMemBlock = size_t(512) << 20, kMemCache = size_t(2) << 30;
 struct MemBlock {
@@ -52,49 +60,133 @@ struct MemBlock {
     size_t bytes;
     int    dev;
 };
-std::mutex           g_mem_mu;
-std::deque<MemBlock> g_mem;  // oldest first
-size_t               g_mem_bytes = 0;
+struct MemCache {
+    std::mutex           mu;      // not held across a CUDA call
+    std::deque<MemBlock> blocks;  // oldest first
+    size_t               bytes = 0;
+    std::map<int, void *> anchor;  // the 512 bytes that stay, per device
+
+    // takes the oldest blocks (of device dev, or of all: dev < 0) until at most `keep` bytes are cached
+    std::vector<void *> drop(int dev, size_t keep) {
+        std::vector<void *> out;
+        for (auto it = blocks.begin(); it != blocks.end() && bytes > keep;) {
+            if (dev >= 0 && it->dev != dev) {
+                ++it;
+                continue;
+            }
+            bytes -= it->bytes;
+            out.push_back(it->p);
+            it = blocks.erase(it);
+        }
+        return out;
+    }
+};
+MemCache &mem_cache() {  // never destroyed: whatever closes last may still give blocks to it
+    static MemCache *c = new MemCache;
+    return *c;
+}
+thread_local int                   t_scopes = 0;  // open MemScopes of this thread, and what they hold
+thread_local std::vector<MemBlock> t_held;
 
 size_t mem_round(size_t n) {
     const size_t unit = n <= (1u << 16) ? 512 : n <= (1u << 20) ? (1u << 14) : (1u << 20);
     return (n + unit - 1) / unit * unit;
 }
-// drops the oldest blocks (of device dev, or of all: dev < 0) until at most `keep` bytes are cached
-void mem_drop(int dev, size_t keep) {
-    for (auto it = g_mem.begin(); it != g_mem.end() && g_mem_bytes > keep;) {
-        if (dev >= 0 && it->dev != dev) {
-            ++it;
-            continue;
-        }
-        g_mem_bytes -= it->bytes;
-        cudaFree(it->p);
-        it = g_mem.erase(it);
+bool mem_free(void *p) {
+    if (cudaFree(p) == cudaSuccess) return true;
+    cudaGetLastError();  // not left for the check of this thread's next launch
+    return false;
+}
+void *mem_small() {
+    void *p = nullptr;
+    if (cudaMalloc(&p, 512) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+// waits for everything queued on device dev
+bool mem_wait(int dev) {
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    bool known;
+    {
+        std::lock_guard<std::mutex> lk(mem_cache().mu);
+        known = mem_cache().anchor.count(dev) != 0;
     }
+    if (!known) {
+        void *a = mem_small();
+        bool  mine = false;
+        if (a) {
+            std::lock_guard<std::mutex> lk(mem_cache().mu);
+            mine = mem_cache().anchor.emplace(dev, a).second;
+        }
+        if (a && !mine) mem_free(a);
+    }
+    void      *p = mem_small();
+    const bool ok = p && mem_free(p);
+    if (cur != dev) cudaSetDevice(cur);
+    return ok;
+}
+// blocks of one device into the cache, or back to the driver
+void mem_release(const std::vector<MemBlock> &in) {
+    if (in.empty()) return;
+    const bool          ok = mem_wait(in[0].dev);
+    std::vector<void *> out;
+    {
+        MemCache                   &c = mem_cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        for (const MemBlock &b : in) {
+            if (!ok || b.bytes > kMemBlock) {
+                out.push_back(b.p);
+                continue;
+            }
+            c.blocks.push_back(b);
+            c.bytes += b.bytes;
+        }
+        for (void *p : c.drop(-1, kMemCache)) out.push_back(p);
+    }
+    for (void *p : out) mem_free(p);
 }
 }  // namespace
+
+mdp_mem_scope::mdp_mem_scope() { t_scopes++; }
+mdp_mem_scope::~mdp_mem_scope() {
+    if (--t_scopes > 0) return;
+    std::vector<MemBlock> in;
+    in.swap(t_held);
+    while (!in.empty()) {  // device by device
+        const int dev = in[0].dev;
+        auto      mid = std::stable_partition(in.begin(), in.end(), [&](const MemBlock &b) { return b.dev == dev; });
+        mem_release(std::vector<MemBlock>(in.begin(), mid));
+        in.erase(in.begin(), mid);
+    }
+}
 
 int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
     const size_t want = mem_round(nbytes);
     *p = nullptr;
     *got = 0;
     MDP_CUDA(cudaGetDevice(dev));
-    std::lock_guard<std::mutex> lk(g_mem_mu);
-    auto best = g_mem.end();
-    for (auto it = g_mem.begin(); it != g_mem.end(); ++it)
-        if (it->dev == *dev && it->bytes >= want && want >= it->bytes / 4 * 3 && (best == g_mem.end() || it->bytes < best->bytes))
-            best = it;
-    if (best != g_mem.end()) {
-        *p = best->p;
-        *got = best->bytes;
-        g_mem_bytes -= best->bytes;
-        g_mem.erase(best);
-        return MDP_OK;
+    {
+        MemCache                   &c = mem_cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        auto                        best = c.blocks.end();
+        for (auto it = c.blocks.begin(); it != c.blocks.end(); ++it)
+            if (it->dev == *dev && it->bytes >= want && want >= it->bytes / 4 * 3 &&
+                (best == c.blocks.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != c.blocks.end()) {
+            *p = best->p;
+            *got = best->bytes;
+            c.bytes -= best->bytes;
+            c.blocks.erase(best);
+            return MDP_OK;
+        }
     }
     cudaError_t e = cudaMalloc(p, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        mem_drop(*dev, 0);
+        mdp_mem_trim(*dev);
         e = cudaMalloc(p, want);
     }
     if (e != cudaSuccess) {
@@ -108,27 +200,17 @@ int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
 }
 
 void mdp_mem_put(void *p, size_t bytes, int dev) {
-    int cur = dev;
-    cudaGetDevice(&cur);
-    if (cur != dev) cudaSetDevice(dev);
-    // what was queued on the block is over before anyone can take it again
-    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
-    {
-        std::lock_guard<std::mutex> lk(g_mem_mu);
-        if (!ok || bytes > kMemBlock) {
-            cudaFree(p);
-        } else {
-            g_mem.push_back(MemBlock{p, bytes, dev});
-            g_mem_bytes += bytes;
-            mem_drop(-1, kMemCache);
-        }
-    }
-    if (cur != dev) cudaSetDevice(cur);
+    if (t_scopes > 0) t_held.push_back(MemBlock{p, bytes, dev});
+    else mem_release({MemBlock{p, bytes, dev}});
 }
 
 void mdp_mem_trim(int dev) {
-    std::lock_guard<std::mutex> lk(g_mem_mu);
-    mem_drop(dev, 0);
+    std::vector<void *> out;
+    {
+        std::lock_guard<std::mutex> lk(mem_cache().mu);
+        out = mem_cache().drop(dev, 0);
+    }
+    for (void *p : out) mem_free(p);
 }
 
 // ============================================================== context
@@ -174,9 +256,12 @@ extern "C" int mdp_context_trim(mdp_context *ctx) {
     if (!ctx) return MDP_EINVAL;
     MDP_CUDA(cudaSetDevice(ctx->device));
     MDP_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (DevBuf &b : ctx->ws) b.release();
-    ctx->scratch.release();
-    ctx->scratch2.release();
+    {
+        mdp_mem_scope one_wait;
+        for (DevBuf &b : ctx->ws) b.release();
+        ctx->scratch.release();
+        ctx->scratch2.release();
+    }
     mdp_mem_trim(ctx->device);
     return MDP_OK;
 }
@@ -192,6 +277,7 @@ extern "C" void mdp_context_destroy(mdp_context *ctx) {
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     for (int i = 0; i < 5; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
+    mdp_mem_scope one_wait;
     delete ctx;
 }
 
@@ -556,7 +642,10 @@ extern "C" int mdp_pointing_create(mdp_context *ctx, int64_t m, int nnz, const i
     return mdp_pointing_create_ex(ctx, m, nnz, d_gindices, d_values, nullptr, out);
 }
 
-extern "C" void mdp_pointing_destroy(mdp_pointing *A) { delete A; }
+extern "C" void mdp_pointing_destroy(mdp_pointing *A) {
+    mdp_mem_scope one_wait;
+    delete A;
+}
 
 extern "C" int mdp_pointing_shape(const mdp_pointing *A, int64_t *lcount, int *trash_pix, int64_t *n_map,
                                   int *triplet_layout) {

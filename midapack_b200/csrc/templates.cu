@@ -371,7 +371,10 @@ extern "C" int mdp_templates_create(mdp_context *ctx, const mdp_template_scan *s
     return MDP_OK;
 }
 
-extern "C" void mdp_templates_destroy(mdp_templates *T) { delete T; }
+extern "C" void mdp_templates_destroy(mdp_templates *T) {
+    mdp_mem_scope one_wait;
+    delete T;
+}
 
 extern "C" int mdp_templates_samples(const mdp_templates *T, int64_t *m, int64_t *n_amplitudes) {
     if (!T) return MDP_EINVAL;

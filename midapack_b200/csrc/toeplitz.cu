@@ -1839,7 +1839,10 @@ extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *
     return MDP_OK;
 }
 
-extern "C" void mdp_noise_destroy(mdp_noise *N) { delete N; }
+extern "C" void mdp_noise_destroy(mdp_noise *N) {
+    mdp_mem_scope one_wait;
+    delete N;
+}
 
 extern "C" int mdp_noise_tile(const mdp_noise *N, int *fft_size, int *cluster_ctas, int64_t *n_tiles) {
     if (!N) return MDP_EINVAL;
