@@ -137,8 +137,8 @@ __device__ __forceinline__ double ld_sample(const double *p) {
 // sample n of the window, less the block mean; zero outside the block
 template <typename T>
 __device__ __forceinline__ T sample(const Tile<T> &tl, int n) {
-    const int i = tl.o + n;
-    return (unsigned) i < (unsigned) tl.len ? ld_sample(tl.in + i) - tl.mu : (T) 0;
+    const unsigned i = (unsigned) tl.o + (unsigned) n;  // past 2^31 in the last tile of the longest blocks
+    return i < (unsigned) tl.len ? ld_sample(tl.in + i) - tl.mu : (T) 0;
 }
 // the same of a window inside its block: point j0 + n, n known at compile time
 template <typename T>
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256, rt_col_ctas<T>()) rt_cols_kernel(RArgs<T>
     int           spec;
     if (!tile_of(a, a.item0 + li, tl, spec)) return;
     auto *Y = a.Y + (int64_t) li * M;
-    if (tl.o >= 0 && tl.o + 2 * M <= tl.len)
+    if (tl.o >= 0 && tl.o <= tl.len - 2 * M)
         cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample_in(tl, j0, n), sample_in(tl, j0, n + M)); });
     else
         cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample(tl, j0 + n), sample(tl, j0 + n + M)); });
