@@ -939,15 +939,22 @@ __global__ void __launch_bounds__(32) bin_chunk_scatter_kernel(const int32_t *__
 // constant for setting up and adding up its map (PT_FIXED rows' worth): a
 // wave begun for a few CTAs costs as much as a full one.  A function of the row counts alone,
 // so that the sums are the same on every device.  (Slices of a fixed power of two of rows
-// left 1.7 waves for 4 x 2^20 rows on 49152 pixels: 47 us.)
+// left 1.7 waves for 4 x 2^20 rows on 49152 pixels: 47 us.)  Measured, us, on maps of 1024 x 768 pixels:
+//                          2 x 2^20 rows   16 x 2^20   16 x 2^22
+// as below                     23.3           121         438
+// PT_FIXED 0, 64, 768      31.2 23.3 23.4  162 162 149  450 449 416
+// no c above 3                 31.6           122         438
+// k = 1 alone                  31.9           158         614
+// no k above 4                 23.2           122         416
 #define PT_WAVE (4 * 148)
 #define PT_FIXED 192
 static std::vector<int32_t> pt_groups(const std::vector<int64_t> &start) {
     const int64_t        nb = (int64_t) start.size() - 1, total = std::max<int64_t>(start[nb], 1);
     std::vector<int32_t> best, g(nb);
     double               best_cost = 0.0;
-    for (int kc : {103, 203, 303, 403, 603, 803, 1203, 1603, 108, 208, 408, 132, 232}) {
-        const int64_t k = kc / 100, c = kc % 100;
+    constexpr struct { int64_t k, c; } tries[] = {{1, 3}, {2, 3}, {3, 3}, {4, 3}, {6, 3}, {8, 3}, {12, 3}, {16, 3},
+                                                  {1, 8}, {2, 8}, {4, 8}, {1, 32}, {2, 32}};
+    for (const auto [k, c] : tries) {
         const int64_t warp_rows = std::max<int64_t>(total / (PT_WAVE * PT_WARPS * k), 128);
         int64_t       ctas = 0, alone = 0, longest = 1;
         for (int64_t b = 0; b < nb; b++) {
