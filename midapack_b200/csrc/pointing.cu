@@ -777,6 +777,10 @@ extern "C" int mdp_matvec(mdp_context *ctx, const mdp_pointing *A, const double 
 }
 
 // ============================================================== x = P^T y
+// Clears the map for the atomics, in the chain of kernels (a memset ends it: solve of 2^18 samples on 6912
+// pixels 2.99 against 3.12 ms).  Maps of up to PT_SET_MAX entries are set by the driver within the
+// stream's command: P^T of 758 rows and 117 pixels 13.0 against 14.3 us, of 192 pixels 14.3 both ways.
+#define PT_SET_MAX 512
 __global__ void pt_zero_kernel(double *__restrict__ x, int64_t n) {
     chain_next();
     chain_wait();
@@ -1300,8 +1304,12 @@ int mdp_trmatvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d
         // every map entry is written by its bin's slice or by the partial sums
         return trmatvec_slices<double, double>(ctx, A, A->values, d_y, d_x);
     }
-    MDP_CUDA(launch_chained(pt_zero_kernel, grid_for(A->n_map(), 256, ctx->sm_count * 8), 256, 0, ctx->stream, d_x, A->n_map()));
-    MDP_CHECK_LAUNCH(ctx);
+    if (A->n_map() <= PT_SET_MAX) {
+        MDP_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * A->n_map(), ctx->stream));
+    } else {
+        MDP_CUDA(launch_chained(pt_zero_kernel, grid_for(A->n_map(), 256, ctx->sm_count * 8), 256, 0, ctx->stream, d_x, A->n_map()));
+        MDP_CHECK_LAUNCH(ctx);
+    }
     if (A->triplet && !aligned16(A->values, d_y)) {
         trmatvec_triplet_scalar_kernel<<<grid_for(A->m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
                 A->off.as<int32_t>(), A->values, d_y, d_x, A->m);
