@@ -312,8 +312,9 @@ __device__ __forceinline__ void chunk_mean(const mdp_chunks &c, double acc) {
 
 // window of a right-angle tile (rtile.cu)
 struct alignas(16) mdp_rtile {
-    int64_t start;             // first row of the tile's block
-    int32_t o, len, e;         // window start relative to it, block length, outputs of the tile
+    int64_t start;             // row of the window's first sample (before the block in its first tile)
+    int32_t lo, cnt;           // samples lo <= n < lo + cnt lie in the block
+    int32_t e;                 // outputs of the tile
     int32_t spec, blk, unused; // spectrum, block
 };
 

@@ -62,12 +62,11 @@ template <typename G> struct alignas(2 * sizeof(Pr<G>)) REnt {  // a complex val
     Pr<G> x, y;
 };
 
-// where a tile's samples lie
+// a tile's window: sample n is in[n] for lo <= n < lo + cnt and zero outside the block; output n is out[n]
 template <typename T> struct Tile {
-    const T *in;   // the block's first sample
+    const T *in;
     T       *out;
-    int      o;    // window start relative to the block
-    int      len;  // block length
+    int      lo, cnt;
     int      e;    // outputs of the tile inside the block
     T        mu;
 };
@@ -114,8 +113,8 @@ __device__ __forceinline__ bool tile_of(const RArgs<T> &a, int64_t item, Tile<T>
     const int64_t bs = (int64_t) (((uint64_t) (uint32_t) d0.y << 32) | (uint32_t) d0.x) + col * a.col_stride;
     tl.in = a.vin + bs;
     tl.out = a.vout + bs;
-    tl.o = d0.z;
-    tl.len = d0.w;
+    tl.lo = d0.z;
+    tl.cnt = d0.w;
     tl.e = d1.x;
     spec = d1.y;
     chain_wait();  // the records above are the plan's own; all else may come from the kernel before
@@ -137,20 +136,19 @@ __device__ __forceinline__ double ld_sample(const double *p) {
 // sample n of the window, less the block mean; zero outside the block
 template <typename T>
 __device__ __forceinline__ T sample(const Tile<T> &tl, int n) {
-    const unsigned i = (unsigned) tl.o + (unsigned) n;  // past 2^31 in the last tile of the longest blocks
-    return i < (unsigned) tl.len ? ld_sample(tl.in + i) - tl.mu : (T) 0;
+    return (unsigned) (n - tl.lo) < (unsigned) tl.cnt ? ld_sample(tl.in + n) - tl.mu : (T) 0;
 }
 // the same of a window inside its block: point j0 + n, n known at compile time
 template <typename T>
 __device__ __forceinline__ T sample_in(const Tile<T> &tl, int j0, int n) {
-    return ld_sample(tl.in + (tl.o + j0) + n) - tl.mu;
+    return ld_sample(tl.in + j0 + n) - tl.mu;
 }
 __device__ __forceinline__ double sample(const RowSrc &r, int n) {
     return n < r.lambda ? __ldg(r.T + n) : (r.M2 - n < r.lambda ? -__ldg(r.T + (r.M2 - n)) : 0.0);
 }
 template <typename T>
 __device__ __forceinline__ void put(const Tile<T> &tl, int halo, int n, T v) {
-    if ((unsigned) (n - halo) < (unsigned) tl.e) tl.out[tl.o + n] = v;
+    if ((unsigned) (n - halo) < (unsigned) tl.e) tl.out[n] = v;
 }
 template <typename T>
 __device__ __forceinline__ CP<typename LaneOf<T>::Tag> point(T x, T y) {
@@ -471,7 +469,7 @@ __global__ void __launch_bounds__(256, rt_col_ctas<T>()) rt_cols_kernel(RArgs<T>
     int           spec;
     if (!tile_of(a, a.item0 + li, tl, spec)) return;
     auto *Y = a.Y + (int64_t) li * M;
-    if (tl.o >= 0 && tl.o <= tl.len - 2 * M)
+    if (tl.cnt == 2 * M)
         cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample_in(tl, j0, n), sample_in(tl, j0, n + M)); });
     else
         cols_forward<T, M1>(a, part, Y, [&](int j0, int n) { return point(sample(tl, j0 + n), sample(tl, j0 + n + M)); });
@@ -629,10 +627,13 @@ int rtile_build(mdp_context *ctx, mdp_noise *N, mdp_tile_plan &P, bool spectra) 
         std::vector<mdp_rtile> tiles;
         const int64_t          E = P.fft_n - 2LL * (N->lambda - 1);
         for (int b = 0; b < N->nb; b++)
-            for (int64_t o = 0; o < N->h_n[b]; o += E)
-                tiles.push_back(mdp_rtile{N->h_idv[b], (int32_t) (o - (N->lambda - 1)), N->h_n[b],
+            for (int64_t o = 0; o < N->h_n[b]; o += E) {
+                const int64_t w = o - (N->lambda - 1), lo = std::max<int64_t>(-w, 0);
+                tiles.push_back(mdp_rtile{N->h_idv[b] + w, (int32_t) lo,
+                                          (int32_t) (std::min<int64_t>(N->h_n[b] - w, P.fft_n) - lo),
                                           (int32_t) std::min<int64_t>(E, N->h_n[b] - o), N->h_spec.empty() ? 0 : N->h_spec[b],
                                           b, 0});
+            }
         MDP_TRY(P.tile_start.alloc(sizeof(mdp_rtile) * std::max<size_t>(tiles.size(), 1)));
         if (!tiles.empty())
             MDP_CUDA(cudaMemcpy(P.tile_start.p, tiles.data(), sizeof(mdp_rtile) * tiles.size(), cudaMemcpyHostToDevice));
