@@ -345,6 +345,7 @@ int mdp_ecg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
 extern "C" int mdp_ecg_solve(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const double *d_signal,
                              const double *d_noise, const mdp_ecg_params *params, double *d_x, int32_t *d_lstid,
                              double *d_cond, int32_t *d_hits, double *h_res_rel, mdp_solve_info *info) {
+    mdp_mem_scope one_wait;
     if (!ctx || !A || !N || !d_signal || !d_noise || !params || !d_x) {
         mdp_set_error("mdp_ecg_solve: invalid arguments");
         return MDP_EINVAL;

@@ -102,8 +102,8 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 int  mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev);
 void mdp_mem_put(void *p, size_t bytes, int dev);
 void mdp_mem_trim(int dev);  // gives the device's cached blocks back to the driver
-// what a thread releases inside it enters the cache at its end, after one wait (for destroying
-// objects of many buffers, not for code that allocates)
+// what a thread releases inside it enters the cache at its end (or from 64 MB on), after one wait for all: for
+// calls with many temporaries and for destroying objects, as the first local of the function
 struct mdp_mem_scope {
     mdp_mem_scope();
     ~mdp_mem_scope();

@@ -802,6 +802,7 @@ extern "C" int mdp_gls_solve_multi(mdp_context *ctx, mdp_pointing *A, const mdp_
                                    int signal_col, const mdp_multi_params *params, double *d_x, int32_t *d_lstid,
                                    double *d_cond, int32_t *d_hits, mdp_multi_col_info *col_info,
                                    mdp_multi_info *info) {
+    mdp_mem_scope one_wait;
     if (!ctx || !A || !Nc || nrhs < 1 || !d_noise || noise_stride < A->m || !params || !d_x || !col_info ||
         params->tol <= 0.0 || params->inner_tol <= 0.0 || params->inner_maxiter < 1 || params->maxiter < 1 ||
         (signal_col >= 0 && !d_signal) || signal_col >= nrhs) {

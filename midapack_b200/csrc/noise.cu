@@ -696,6 +696,7 @@ extern "C" int mdp_apod_window(mdp_context *ctx, int lambda, int apod, double *d
 
 extern "C" int mdp_periodogram(mdp_context *ctx, int nb, const int32_t *h_n, const double *d_noise, double fsamp,
                                double *d_psd) {
+    mdp_mem_scope one_wait;
     if (!ctx || nb < 1 || !h_n || !d_noise || !d_psd || !(fsamp > 0.0) || !std::isfinite(fsamp)) {
         mdp_set_error("mdp_periodogram: bad argument");
         return MDP_EINVAL;
@@ -746,6 +747,7 @@ extern "C" int mdp_periodogram(mdp_context *ctx, int nb, const int32_t *h_n, con
 
 extern "C" int mdp_noise2invtt(mdp_context *ctx, int nb, const int32_t *h_n, const double *d_noise, int lambda,
                                double fsamp, int apod, double *d_invtt, double *h_params, int32_t *h_evals) {
+    mdp_mem_scope one_wait;
     if (!ctx || nb < 1 || !h_n || !d_noise || !d_invtt || lambda < 1 || !(fsamp > 0.0) || !std::isfinite(fsamp)) {
         mdp_set_error("mdp_noise2invtt: bad argument");
         return MDP_EINVAL;

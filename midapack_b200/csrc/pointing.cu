@@ -85,8 +85,10 @@ MemCache &mem_cache() {  // never destroyed: whatever closes last may still give
     static MemCache *c = new MemCache;
     return *c;
 }
-thread_local int                   t_scopes = 0;  // open MemScopes of this thread, and what they hold
+thread_local int                   t_scopes = 0;  // open scopes of this thread, and what they hold
 thread_local std::vector<MemBlock> t_held;
+thread_local size_t                t_held_bytes = 0;
+constexpr size_t kMemHeld = size_t(64) << 20;
 
 size_t mem_round(size_t n) {
     const size_t unit = n <= (1u << 16) ? 512 : n <= (1u << 20) ? (1u << 14) : (1u << 20);
@@ -149,17 +151,21 @@ void mem_release(const std::vector<MemBlock> &in) {
 }
 }  // namespace
 
-mdp_mem_scope::mdp_mem_scope() { t_scopes++; }
-mdp_mem_scope::~mdp_mem_scope() {
-    if (--t_scopes > 0) return;
+// what the thread's scopes hold, device by device
+static void mem_flush() {
     std::vector<MemBlock> in;
     in.swap(t_held);
-    while (!in.empty()) {  // device by device
+    t_held_bytes = 0;
+    while (!in.empty()) {
         const int dev = in[0].dev;
         auto      mid = std::stable_partition(in.begin(), in.end(), [&](const MemBlock &b) { return b.dev == dev; });
         mem_release(std::vector<MemBlock>(in.begin(), mid));
         in.erase(in.begin(), mid);
     }
+}
+mdp_mem_scope::mdp_mem_scope() { t_scopes++; }
+mdp_mem_scope::~mdp_mem_scope() {
+    if (--t_scopes == 0) mem_flush();
 }
 
 int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
@@ -200,8 +206,13 @@ int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
 }
 
 void mdp_mem_put(void *p, size_t bytes, int dev) {
-    if (t_scopes > 0) t_held.push_back(MemBlock{p, bytes, dev});
-    else mem_release({MemBlock{p, bytes, dev}});
+    if (t_scopes == 0) {
+        mem_release({MemBlock{p, bytes, dev}});
+        return;
+    }
+    t_held.push_back(MemBlock{p, bytes, dev});
+    t_held_bytes += bytes;
+    if (t_held_bytes > kMemHeld) mem_flush();
 }
 
 void mdp_mem_trim(int dev) {
@@ -639,6 +650,7 @@ int mdp_pointing_create_ex(mdp_context *ctx, int64_t m, int nnz, const int32_t *
 
 extern "C" int mdp_pointing_create(mdp_context *ctx, int64_t m, int nnz, const int32_t *d_gindices,
                                    const double *d_values, mdp_pointing **out) {
+    mdp_mem_scope one_wait;
     return mdp_pointing_create_ex(ctx, m, nnz, d_gindices, d_values, nullptr, out);
 }
 

@@ -960,6 +960,7 @@ int mdp_pcg_run(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const dou
 extern "C" int mdp_gls_solve(mdp_context *ctx, mdp_pointing *A, const mdp_noise *N, const double *d_signal,
                              const double *d_noise, const mdp_solve_params *params, double *d_x, int32_t *d_lstid,
                              double *d_cond, int32_t *d_hits, double *h_res_rel, mdp_solve_info *info) {
+    mdp_mem_scope one_wait;
     if (!ctx || !A || !N || !d_signal || !d_noise || !params || !d_x) {
         mdp_set_error("mdp_gls_solve: invalid arguments");
         return MDP_EINVAL;
@@ -1036,6 +1037,7 @@ extern "C" int mdp_gls_solve_mixed(mdp_context *ctx, mdp_pointing *A, const mdp_
                                    const double *d_noise, const mdp_solve_params *params, double inner_tol,
                                    int inner_maxiter, double *d_x, int32_t *d_lstid, double *d_cond, int32_t *d_hits,
                                    double *h_res_rel, mdp_solve_info *info) {
+    mdp_mem_scope one_wait;
     if (!ctx || !A || !Nc || !d_signal || !d_noise || !params || !d_x || inner_tol <= 0.0 || inner_maxiter < 1) {
         mdp_set_error("mdp_gls_solve_mixed: invalid arguments");
         return MDP_EINVAL;

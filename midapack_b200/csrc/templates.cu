@@ -416,6 +416,7 @@ extern "C" int mdp_gls_solve_templates(mdp_context *ctx, mdp_pointing *A, const 
                                        const double *d_signal, const double *d_noise, const mdp_solve_params *params,
                                        double *d_x, int32_t *d_lstid, double *d_cond, int32_t *d_hits,
                                        double *h_res_rel, mdp_solve_info *info) {
+    mdp_mem_scope one_wait;
     if (!ctx || !A || !N || !T || !d_signal || !d_noise || !params || !d_x) {
         mdp_set_error("mdp_gls_solve_templates: invalid arguments");
         return MDP_EINVAL;

@@ -1714,6 +1714,7 @@ static int launch_tiles(mdp_context *ctx, const mdp_noise *N, const mdp_tile_pla
 
 extern "C" int mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *h_idv, const int32_t *h_n, int lambda,
                                 const double *h_T, mdp_noise **out) {
+    mdp_mem_scope one_wait;
     if (!ctx || !out || nb_blocks <= 0 || !h_idv || !h_n || !h_T || lambda < 1) {
         mdp_set_error("mdp_noise_create: invalid arguments");
         return MDP_EINVAL;
