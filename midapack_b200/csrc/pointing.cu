@@ -790,8 +790,10 @@ extern "C" int mdp_matvec(mdp_context *ctx, const mdp_pointing *A, const double 
 
 // ============================================================== x = P^T y
 // Clears the map for the atomics, in the chain of kernels (a memset ends it: solve of 2^18 samples on 6912
-// pixels 2.99 against 3.12 ms).  Maps of up to PT_SET_MAX entries are set by the driver within the
-// stream's command: P^T of 758 rows and 117 pixels 13.0 against 14.3 us, of 192 pixels 14.3 both ways.
+// pixels 2.99 against 3.12 ms).  Maps of up to PT_SET_MAX entries, which the driver sets within the stream's
+// command, are left to a memset while their atomics are short, at most 16 rows an entry: P^T of 758 rows
+// on 117 pixels 12.8 us alone and 6.1 among others, with the kernel 14.2 and 6.5; of 12000 rows on as many 15.9
+// and 8.2 against 17.4 and 6.5; of 192 pixels the same both ways.
 #define PT_SET_MAX 512
 __global__ void pt_zero_kernel(double *__restrict__ x, int64_t n) {
     chain_next();
@@ -1316,7 +1318,7 @@ int mdp_trmatvec_launch(mdp_context *ctx, const mdp_pointing *A, const double *d
         // every map entry is written by its bin's slice or by the partial sums
         return trmatvec_slices<double, double>(ctx, A, A->values, d_y, d_x);
     }
-    if (A->n_map() <= PT_SET_MAX) {
+    if (A->n_map() <= PT_SET_MAX && A->m <= 16 * A->n_map()) {
         MDP_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * A->n_map(), ctx->stream));
     } else {
         MDP_CUDA(launch_chained(pt_zero_kernel, grid_for(A->n_map(), 256, ctx->sm_count * 8), 256, 0, ctx->stream, d_x, A->n_map()));
