@@ -1250,6 +1250,11 @@ static int ceil_log2(int64_t v) {
     return b;
 }
 
+// 40 to 80 us for the host to queue the launches of a short trial
+__global__ void tune_delay_kernel() {
+    for (int i = 0; i < 40; i++) __nanosleep(1000);
+}
+
 template <typename T>
 static int tune_plan(mdp_context *ctx, const mdp_noise *N, const std::vector<TileCand> &cands, TileCand *best) {
     // sample: whole blocks from the start, at most 2^24 rows (one long block is cut there)
@@ -1295,18 +1300,24 @@ static int tune_plan(mdp_context *ctx, const mdp_noise *N, const std::vector<Til
         mdp_tile_plan P;
         if ((rc = build_plan<T>(ctx, &S, P, c, false))) break;
         if ((rc = launch_tiles<T>(ctx, &S, P, in.as<T>(), out.as<T>(), S.means.as<double>()))) break;  // warm-up
-        float ms = 1e30f;  // best of three trials of two applications
-        for (int trial = 0; trial < 3 && rc == MDP_OK; trial++) {
+        // Best of three trials of two applications.  Up to 2^20 rows an application is shorter than its launches
+        // take on the host, which would then be what is compared: best of two trials of four, queued
+        // behind a delay (10 x 269 samples, half bandwidth 135, FP64: without it 10.5 us in most processes, now 8.5).
+        const bool small = rows <= (1 << 20);
+        const int  reps = small ? 4 : 2;
+        float      ms = 1e30f;
+        for (int trial = small ? 1 : 0; trial < 3 && rc == MDP_OK; trial++) {
             float t = 0.f;
+            if (small) tune_delay_kernel<<<1, 1, 0, ctx->stream>>>();
             cudaEventRecord(e0, ctx->stream);
-            for (int r = 0; r < 2 && rc == MDP_OK; r++)
+            for (int r = 0; r < reps && rc == MDP_OK; r++)
                 rc = launch_tiles<T>(ctx, &S, P, in.as<T>(), out.as<T>(), S.means.as<double>());
             cudaEventRecord(e1, ctx->stream);
             if (rc == MDP_OK && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t, e0, e1) != cudaSuccess)) {
                 rc = MDP_ECUDA;
                 mdp_set_error("tile autotuner: %s", cudaGetErrorString(cudaGetLastError()));
             }
-            ms = std::min(ms, t);
+            ms = std::min(ms, t / (float) reps);
         }
         if (rc) break;
         if (ms < bestt) {
@@ -1365,13 +1376,15 @@ static int choose_plan(mdp_context *ctx, const mdp_noise *N, TileCand *out, int 
     });
     *out = cands[0];
     if (forced || !tune || cands.size() == 1) return MDP_OK;
-    // screen: tiles at least an eighth useful and not longer than twice the block plus the halo (a quarter left
-    // out the tile of 2048 samples at half bandwidth 900, the faster one for 4 x 12000: 12.7 against 14.9 us)
+    // screen: the cost model's choice, and tiles at least an eighth useful and not longer than twice the block
+    // plus the halo (a quarter left out the tile of 2048 samples at half bandwidth 900, the faster one for 4 x 12000: 12.7
+    // against 14.9 us at the time; without the model's choice 21 blocks of 98 to 194 samples, 98, FP32 took a
+    // one-kernel tile of 10.5 us, where the shortest right-angle tile takes 6.9)
     std::vector<TileCand> screen;
     uint64_t              bits = 0;
     for (const TileCand &c : cands) {
         const int64_t Nn = cand_N(c), E = cand_E(c, N->lambda);
-        if (E * 8 < Nn || E > 2 * std::max<int64_t>(N->max_block, 1) + 2LL * N->lambda) continue;
+        if (&c != &cands[0] && (E * 8 < Nn || E > 2 * std::max<int64_t>(N->max_block, 1) + 2LL * N->lambda)) continue;
         screen.push_back(c);
         bits |= cand_bit(c) | (E * 4 < Nn ? 0 : cand_bit(c) << 32);
     }
