@@ -18,7 +18,7 @@
 // Before, each run of equal lengths went through on its own: four passes for two filters
 // (one of them the inverse transform's, unused), radix-2 stages with a barrier each, and
 // the launches of a 2^19-point transform on 128 CTAs.  32 blocks of 100002 to 200003
-// samples: 9.0 ms, 13-17 ms with the allocations between calls; now 0.71 ms, bound by the
+// samples: 9.0 ms, 13-17 ms with the allocations between calls; now 0.72 ms, bound by the
 // CTAs' load, exchange and store phases at two CTAs an SM.
 #include <algorithm>
 #include <cmath>
@@ -38,7 +38,7 @@ struct PsdBlock {
     int64_t at;      // first sample
     int64_t out;     // first density
     int     n, filt; // samples; chirp filter of the group (-1: L = n, none)
-    double  inv_stt, scale;
+    double  inv_stt, inv_stt_lo, scale;  // 1 / sum (t - (n-1)/2)^2 in two parts
 };
 
 struct PsdArgs {
@@ -49,7 +49,7 @@ struct PsdArgs {
     const double2  *tw1;    // [16][256] W_4096^(q k)
     const double2  *tw2;    // [16][16]  W_256^(c k)
     const double2  *tw4k;   // [4096]    W_4096^e
-    const double   *sums;   // [cnt][2] sum x, sum (t - (n-1)/2) x
+    const double4  *line;   // [cnt] least-squares line: mean and slope in two parts each
     double2        *buf;    // [cnt + nfilt][n1][4096]
     int             cnt, nfilt, n1;
 };
@@ -72,25 +72,20 @@ __device__ __forceinline__ double2 expi(double turns_pi, double sign) {
     sincospi(turns_pi, &s, &c);
     return make_double2(c, sign * s);
 }
-// a / n for many a and one n: the quotient by the reciprocal and one step of residual correction
-// (Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990), within an
-// ulp of the correctly rounded one, in place of a division each.  With divisions and a 64-bit
-// modulo the columns of 12 blocks and their filters (L = 2^18) took 39 M warp instructions and
-// 86 us, with it 34 M and 74; 32 blocks of 100002 to 200003 samples 0.757 -> 0.711 ms.
+// A length and its reciprocal: the angles pi a / n below are at most a quarter of a turn, so that the rounding
+// of the reciprocal and of a product with it moves them by 2^-54 of a turn at most, and no quotient is formed.  (With
+// a division each and a 64-bit modulo the columns of 12 blocks and their filters, L = 2^18, took 39 M warp
+// instructions and 86 us, without 34 M and 74.)
 struct Recip {
     double n, inv;
-    __device__ __forceinline__ double div(double a) const {
-        const double q = a * inv;
-        return fma(fma(-q, n, a), inv, q);
-    }
 };
 // exp(sign i pi m^2 / n): m^2 < 2^48 less the nearest multiple k of n/2, exactly (multiples of 1/2 below
 // 2^53), so that the angle is at most an eighth of a turn and its rounding as much smaller; then k quarter turns.
 // Amplitudes of 174763 white samples against extended precision: 3.87e-16 with angles of up to a turn, 3.52e-16
-// with these and the window's within a quarter turn (100003 samples 3.26 and 2.82), for 1 % of the time.
+// with these and the window's within a quarter turn (100003 samples 3.26 and 2.82).
 __device__ __forceinline__ double2 chirp1(int m, const Recip &n, double sign) {
     const double  mm = (double) m * (double) m, k = rint(mm * (2.0 * n.inv));
-    const double2 w = expi(n.div(fma(-k, 0.5 * n.n, mm)), 1.0);
+    const double2 w = expi(fma(-k, 0.5 * n.n, mm) * n.inv, 1.0);
     const int     q = (int) k;
     const double  c = q & 1 ? w.y : w.x, s = q & 1 ? w.x : w.y;
     return make_double2((q + 1) & 2 ? -c : c, sign * (q & 2 ? -s : s));
@@ -103,8 +98,30 @@ __global__ void psd_tables_kernel(double2 *tw1, double2 *tw2, double2 *tw4k) {
     tw4k[e] = expi((double) e / 2048.0, -1.0);
 }
 
+// A number as the unevaluated sum of two doubles, for the least-squares line of a block: the same error in
+// the line at every sample falls into the lowest bins, which hold most of 1/f data (12909 samples against extended
+// precision, the line's part alone: plain sums, rounded mean and slope 3.4e-16 of a block's norm on average and up
+// to 3.0e-15, in two parts 3e-17).  The roundings of single samples, and of the sums of a warp's few
+// hundred, average out: those stay plain.
+struct Two {
+    double h, l;
+};
+__device__ __forceinline__ Two operator+(Two a, Two b) {  // two-sum: Knuth, The Art of Computer Programming, vol. 2
+    const double s = a.h + b.h, t = s - a.h;
+    return {s, (a.h - (s - t)) + (b.h - t) + (a.l + b.l)};
+}
+__device__ __forceinline__ double warp_sum(double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ Two warp_sum(Two v) {
+    for (int o = 16; o > 0; o >>= 1)
+        v = v + Two{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)};
+    return v;
+}
+
 // sums of x and (t - (n-1)/2) x over each block: partials, chunk by chunk
-__global__ void __launch_bounds__(kT) psd_sums_kernel(PsdArgs a, double *part) {
+__global__ void __launch_bounds__(kT) psd_sums_kernel(PsdArgs a, Two *part) {
     const PsdBlock b = a.blk[blockIdx.y];
     const double  *x = a.x + b.at;
     const double   c = 0.5 * (double) (b.n - 1);
@@ -115,34 +132,41 @@ __global__ void __launch_bounds__(kT) psd_sums_kernel(PsdArgs a, double *part) {
         s1 += ((double) t - c) * v;
     }
     __shared__ double sh[2][kT / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    }
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
     if ((threadIdx.x & 31) == 0) {
         sh[0][threadIdx.x >> 5] = s0;
         sh[1][threadIdx.x >> 5] = s1;
     }
     __syncthreads();
     if (threadIdx.x < 2) {
-        double v = 0.0;
-        for (int w = 0; w < kT / 32; w++) v += sh[threadIdx.x][w];
+        Two v{0.0, 0.0};
+        for (int w = 0; w < kT / 32; w++) v = v + Two{sh[threadIdx.x][w], 0.0};
         part[((int64_t) blockIdx.y * 2 + threadIdx.x) * gridDim.x + blockIdx.x] = v;
     }
 }
-__global__ void __launch_bounds__(kT) psd_sums_final_kernel(const double *part, int chunks, int n2, double *sums) {
-    const int s = (blockIdx.x * kT + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (s >= n2) return;
-    double v = 0.0;
-    for (int c = lane; c < chunks; c += 32) v += part[(int64_t) s * chunks + c];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sums[s] = v;
+// mean and slope of each block, a warp a block
+__global__ void __launch_bounds__(kT) psd_line_kernel(PsdArgs a, const Two *part, int chunks, double4 *line) {
+    const int i = (blockIdx.x * kT + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= a.cnt) return;
+    Two s[2];
+    for (int q = 0; q < 2; q++) {
+        s[q] = Two{0.0, 0.0};
+        for (int c = lane; c < chunks; c += 32) s[q] = s[q] + part[((int64_t) i * 2 + q) * chunks + c];
+        s[q] = warp_sum(s[q]);
+    }
+    if (lane != 0) return;
+    const PsdBlock b = a.blk[i];
+    const double   n = (double) b.n, m = s[0].h / n, k = s[1].h * b.inv_stt;
+    line[i] = make_double4(m, (fma(-m, n, s[0].h) + s[0].l) / n, k,
+                           fma(s[1].h, b.inv_stt, -k) + (s[1].h * b.inv_stt_lo + s[1].l * b.inv_stt));
 }
 
 // point j of a block's transform input: detrended, windowed, chirped sample; or of a filter
 struct Load {
     const double *x;
-    double        mean, slope, c;
+    double4       line;
+    double        c;
     Recip         rn;       // of n
     int           n, kind;  // 0: samples, 1: chirped samples, 2: filter
     int           L;
@@ -159,8 +183,9 @@ __device__ __forceinline__ C1 point(const Load &l, int j) {
     // (1 - cos(2 pi j / n)) / 2, the angle within a quarter turn of 0 or 1/2 (exact for a power of two)
     const int    h = 2 * min(j, l.n - j);
     const bool   far = 2 * h > l.n;
-    const double w = fma(far ? 0.5 : -0.5, cospi(l.rn.div((double) (far ? l.n - h : h))), 0.5);
-    const double v = (__ldg(l.x + j) - l.mean - l.slope * ((double) j - l.c)) * w;
+    const double w = fma(far ? 0.5 : -0.5, cospi((double) (far ? l.n - h : h) * l.rn.inv), 0.5);
+    const double t = (double) j - l.c;
+    const double v = (fma(-l.line.z, t, __ldg(l.x + j) - l.line.x) - fma(l.line.w, t, l.line.y)) * w;
     if (l.kind == 0) return mk(v, 0.0);
     const double2 ch = chirp1(j, l.rn, -1.0);
     return mk(v * ch.x, v * ch.y);
@@ -193,8 +218,7 @@ __global__ void __launch_bounds__(kT, 2) psd_cols_kernel(PsdArgs a) {
             l.x = a.x + b.at;
             l.n = b.n;
             l.kind = b.filt < 0 ? 0 : 1;
-            l.mean = a.sums[2 * item] / (double) b.n;
-            l.slope = a.sums[2 * item + 1] * b.inv_stt;
+            l.line = a.line[item];
             l.c = 0.5 * (double) (b.n - 1);
         } else {
             l.n = a.fn[item - a.cnt];
@@ -403,8 +427,8 @@ int mdp_psd_blocks(mdp_context *ctx, const std::vector<int> &idx, const int32_t 
             g.nf++;
         }
         // constants of the block, each rounded once
-        const long double dn = n[b], il = 1.0L / (long double) L;
-        blk.push_back(PsdBlock{at[b], out[b], n[b], p2 ? -1 : g.nf - 1, (double) (12.0L / (dn * (dn * dn - 1.0L))),
+        const long double dn = n[b], il = 1.0L / (long double) L, is = 12.0L / (dn * (dn * dn - 1.0L));
+        blk.push_back(PsdBlock{at[b], out[b], n[b], p2 ? -1 : g.nf - 1, (double) is, (double) (is - (long double) (double) is),
                                (double) (8.0L * (p2 ? 1.0L : il * il) / (3.0L * (long double) fsamp * dn))});
         g.cnt++;
         g.chunks = std::max<int>(g.chunks, (int) std::min<int64_t>(((int64_t) n[b] + 4095) / 4096, 256));
@@ -414,11 +438,12 @@ int mdp_psd_blocks(mdp_context *ctx, const std::vector<int> &idx, const int32_t 
     // one buffer: tables, descriptors, the sums of a group and its work arrays
     auto   up = [](size_t b) { return (b + 255) & ~size_t(255); };
     size_t o_blk = up(16 * (2 * 4096 + 256)), o_fn = o_blk + up(sizeof(PsdBlock) * blk.size()), o_part = o_fn + up(4 * fn.size()),
-           o_sum = o_part + up(8 * parts), o_buf = o_sum + up(16 * blk.size());
+           o_line = o_part + up(sizeof(Two) * parts), o_buf = o_line + up(sizeof(double4) * blk.size());
     MDP_TRY(ctx->scratch.alloc(o_buf + work));
     char    *base = ctx->scratch.as<char>();
     double2 *tab = (double2 *) base;
-    double  *part = (double *) (base + o_part), *sums = (double *) (base + o_sum);
+    Two     *part = (Two *) (base + o_part);
+    double4 *line = (double4 *) (base + o_line);
     psd_tables_kernel<<<16, 256, 0, ctx->stream>>>(tab, tab + 8192, tab + 4096);
     MDP_CHECK_LAUNCH(ctx);
     MDP_CUDA(cudaMemcpyAsync(base + o_blk, blk.data(), sizeof(PsdBlock) * blk.size(), cudaMemcpyHostToDevice, ctx->stream));
@@ -433,14 +458,14 @@ int mdp_psd_blocks(mdp_context *ctx, const std::vector<int> &idx, const int32_t 
         a.tw1 = tab;
         a.tw4k = tab + 4096;
         a.tw2 = tab + 8192;
-        a.sums = sums;
+        a.line = line;
         a.buf = (double2 *) (base + o_buf);
         a.cnt = g.cnt;
         a.nfilt = g.nf;
         a.n1 = 1 << (g.ll - 12);
         psd_sums_kernel<<<dim3(g.chunks, g.cnt), kT, 0, ctx->stream>>>(a, part);
         MDP_CHECK_LAUNCH(ctx);
-        psd_sums_final_kernel<<<(2 * g.cnt * 32 + kT - 1) / kT, kT, 0, ctx->stream>>>(part, g.chunks, 2 * g.cnt, sums);
+        psd_line_kernel<<<(g.cnt * 32 + kT - 1) / kT, kT, 0, ctx->stream>>>(a, part, g.chunks, line);
         MDP_CHECK_LAUNCH(ctx);
         const size_t csm = g.ll - 12 > 4 ? kSmem : 0;
         MDP_TRY(launch(ctx, cols_kernel<false>(g.ll - 12), dim3(a.n1, g.cnt + g.nf), csm, a));
