@@ -44,7 +44,8 @@ extern "C" const char *mdp_strerror(int code) {
 // ============================================================== device memory
 // Freed blocks kept for the next allocation of about their size: blocks of up to
 // kMemBlock bytes, kMemCache bytes in all; beyond that the oldest go back to the
-// driver, all of a device's on mdp_context_trim or when the driver is out of memory.
+// driver, all of a device's on mdp_context_trim, with its last context, or when the driver
+// is out of memory.
 // Sizes are rounded up so that blocks fit again; a block is taken for a request of at
 // least three quarters of it.
 //
@@ -65,6 +66,7 @@ struct MemCache {
     std::deque<MemBlock> blocks;  // oldest first
     size_t               bytes = 0;
     std::map<int, void *> anchor;  // the 512 bytes that stay, per device
+    std::map<int, int>    users;   // contexts per device: without one nothing is kept
 
     // takes the oldest blocks (of device dev, or of all: dev < 0) until at most `keep` bytes are cached
     std::vector<void *> drop(int dev, size_t keep) {
@@ -132,13 +134,20 @@ bool mem_wait(int dev) {
 // blocks of one device into the cache, or back to the driver
 void mem_release(const std::vector<MemBlock> &in) {
     if (in.empty()) return;
-    const bool          ok = mem_wait(in[0].dev);
+    const int dev = in[0].dev;
+    bool      keep;
+    {
+        std::lock_guard<std::mutex> lk(mem_cache().mu);
+        keep = mem_cache().users[dev] > 0;
+    }
+    keep = keep && mem_wait(dev);
     std::vector<void *> out;
     {
         MemCache                   &c = mem_cache();
         std::lock_guard<std::mutex> lk(c.mu);
+        keep = keep && c.users[dev] > 0;  // the last context may have gone meanwhile
         for (const MemBlock &b : in) {
-            if (!ok || b.bytes > kMemBlock) {
+            if (!keep || b.bytes > kMemBlock) {
                 out.push_back(b.p);
                 continue;
             }
@@ -224,6 +233,24 @@ void mdp_mem_trim(int dev) {
     for (void *p : out) mem_free(p);
 }
 
+// a context of device dev comes (1) or goes (-1); the last one takes the device's blocks along
+static void mem_user(int dev, int step) {
+    std::vector<void *> out;
+    {
+        MemCache                   &c = mem_cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        c.users[dev] += step;
+        if (c.users[dev] > 0) return;
+        out = c.drop(dev, 0);
+        auto a = c.anchor.find(dev);
+        if (a != c.anchor.end()) {
+            out.push_back(a->second);
+            c.anchor.erase(a);
+        }
+    }
+    for (void *p : out) mem_free(p);
+}
+
 // ============================================================== context
 extern "C" int mdp_context_create(int device, mdp_context **out) {
     if (!out) return MDP_EINVAL;
@@ -251,6 +278,7 @@ extern "C" int mdp_context_create(int device, mdp_context **out) {
         mdp_set_error("cudaMallocHost failed");
         return MDP_ENOMEM;
     }
+    mem_user(device, 1);
     // the side stream here and not on first use, which may be inside a graph capture
     if (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->side_ev[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -288,8 +316,12 @@ extern "C" void mdp_context_destroy(mdp_context *ctx) {
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     for (int i = 0; i < 5; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
-    mdp_mem_scope one_wait;
-    delete ctx;
+    const int dev = ctx->device;
+    {
+        mdp_mem_scope one_wait;
+        delete ctx;
+    }
+    mem_user(dev, -1);
 }
 
 extern "C" int mdp_context_set_stream(mdp_context *ctx, void *cuda_stream) {

@@ -76,3 +76,42 @@ def test_closed_memory_is_taken_after_its_queued_work(gpu_ctx):
     assert torch.allclose(q.view(-1, 3)[:, 0], want, rtol=1e-13)
     Q.close()
     ctx2.close()
+
+
+def test_the_last_context_takes_the_cache_along():
+    """In a process of its own: nothing of the library's stays on the device once its contexts are closed."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch, midapack_b200 as mb
+def used():
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+m = 1 << 24
+def once():
+    idx = (torch.arange(m, device="cuda", dtype=torch.int32) % 5000)[:, None] * 3 + torch.arange(3, device="cuda", dtype=torch.int32)
+    w = torch.ones(3 * m, dtype=torch.float64, device="cuda")
+    y = torch.ones(m, dtype=torch.float64, device="cuda")
+    x = torch.empty(15000, dtype=torch.float64, device="cuda")
+    ctx = mb.Context(0)
+    P = mb.Pointing(ctx, idx.reshape(-1), w, m)
+    P.trmatvec(y, x)
+    P.close()
+    late = mb.Pointing(ctx, idx.reshape(-1), w, m)
+    late.trmatvec(y, x)
+    ctx.close()
+    late.close()          # after the last context: nothing to keep it for
+once()                    # kernels and tables are loaded
+ctx = mb.Context(0)
+ctx.trim()
+ctx.close()
+start = used()
+once()
+print(used() - start)
+"""
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, check=True,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert abs(int(out.stdout.split()[-1])) <= 8 << 20, out.stdout
