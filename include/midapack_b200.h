@@ -48,7 +48,11 @@ void     mdp_context_destroy(mdp_context *ctx);
  * the context's stream).  Device memory that the library gives up (buffers of
  * destroyed objects, temporaries) is kept for its next allocations, up to 2 GiB
  * in blocks of up to 512 MiB for the process; mdp_context_trim gives that of the
- * context's device back to the driver too. */
+ * context's device back to the driver too, and so does destroying the device's last
+ * context.  A call that gives memory up, closing
+ * an object among them, returns after the device has finished what was queued
+ * on it, and does not disturb a stream capture of another thread (thread-local
+ * capture mode). */
 int      mdp_context_trim(mdp_context *ctx);
 /* queue work on an existing cudaStream_t (e.g. the caller's; pass cudaStreamLegacy,
  * i.e. (void *) 1, for the legacy default stream); NULL = a stream of its own */
@@ -87,7 +91,11 @@ int  mdp_trmatvec(mdp_context *ctx, const mdp_pointing *A, const double *d_y, do
 /* ---- inverse noise N^-1: block-diagonal banded symmetric Toeplitz --------
  * (reference: Tpltz/Block, algebra/include/toeplitz/toeplitz.h:152-203)
  * Block b covers rows [h_idv[b], h_idv[b] + h_n[b]) and its first row is
- * h_T[b*lambda .. b*lambda+lambda).  Spectra are computed once here. */
+ * h_T[b*lambda .. b*lambda+lambda).  Spectra are computed once here.
+ * An operator holds work arrays of its own (block means and their counts, the
+ * scratch of its tiles), a pointing too (the partial maps of P^T): calls on one
+ * object, solves among them, must not overlap on the device.  Contexts that share
+ * one order their calls (wait for the stream or an event of the other's). */
 int  mdp_noise_create(mdp_context *ctx, int nb_blocks, const int64_t *h_idv, const int32_t *h_n,
                       int lambda, const double *h_T, mdp_noise **out);
 void mdp_noise_destroy(mdp_noise *N);
@@ -118,7 +126,8 @@ int  mdp_prepare_fp32(mdp_context *ctx, mdp_pointing *A, mdp_noise *N);
  * of M1 x 4096 points reports split_log_m1 = log2(M1) > 0, split_log_m2 = 12 and
  * cluster 0, one of a single row split_log_m1 = 0 and split_log_m2 = log2 of its
  * points (0 for the other one-kernel plans).  The autotuner runs
- * once per precision, band (ceil log2 lambda) and block length class. */
+ * once per precision, band (ceil log2 lambda), block length and row count class and set
+ * of tiles that come into question. */
 int  mdp_noise_plan(mdp_context *ctx, mdp_noise *N, int fp32, int *log2_cta_points, int *cluster_ctas,
                     int *threads, int *tuned, int *split_log_m1, int *split_log_m2);
 /* No counterpart in the reference.  Replaces the tile plan of one precision

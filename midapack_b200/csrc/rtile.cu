@@ -36,7 +36,7 @@
 //
 // Measured against the best of the even/odd-packed plans on a B200 (64 x 2^20 samples,
 // half bandwidth 2^14): FP32 0.93 -> 0.58 ms, error against 64 bits 5.9e-7 -> 2.7e-7; FP64
-// 1.62 -> 1.19 ms, 1.1e-15 -> 8.7e-16.  The row kernel takes half of it: L1 74 % busy in
+// 1.62 -> 1.19 ms, 1.1e-15 -> 8.3e-16.  The row kernel takes half of it: L1 74 % busy in
 // FP32, waiting for its loads in FP64; the columns wait for theirs.  A spectrum from the transform itself takes
 // microseconds where the direct cosine sums took 3.7 ms (half bandwidth 2^13, 2^17 samples).
 #include <algorithm>

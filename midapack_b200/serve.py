@@ -13,7 +13,8 @@ free and its working memory fits the HBM budget (first fit in arrival order,
 so a small request does not wait behind a large one that does not fit yet,
 and a request that waited longer than `max_bypass_s` stops later ones from
 passing it).  Datasets beyond the dataset budget are evicted least recently
-used when not in use.
+used when not in use.  The library's cache of freed device blocks (up to 2 GiB
+a process) comes on top of both budgets.
 
 The scheduler (Server) does not touch the GPU itself: it drives an executor
 with prepare(spec) -> dataset, run(dataset, request) -> Result and
