@@ -197,13 +197,16 @@ def algorithmic_bytes32(ns: int, n_map: int, t32):
 
 
 # DRAM bytes per tile of one N^-1 application, measured with ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum of the three split kernels,
+# (dram__bytes_read.sum + dram__bytes_write.sum of the plan's three kernels,
 # lambda 2^14, 2^20-sample blocks), keyed by (precision, M1, M2); scaled to a
-# launch by the tile count.  256 x 256: 704 tiles in one application; 256 x 512:
+# launch by the tile count.  Split 256 x 256: 704 tiles in one application; 256 x 512:
 # three applications of 160 tiles, the split_pairs_kernel's 1.3 MB taken out
-# (profiles/ninv_split_fp32_256x256_lambda16384.md, operator_p_pt_ninv_dram_2p25.md)
+# (profiles/ninv_split_fp32_256x256_lambda16384.md, operator_p_pt_ninv_dram_2p25.md);
+# right-angle 16 x 4096: 352 (FP32) and 176 (FP64) tiles (profiles/ninv_right_angle.md)
 NINV_TRAFFIC_PER_TILE = {("f32", 256, 256): 1857072128 / 704,
-                         ("f32", 256, 512): (2370306304 - 1314000) / (3 * 160)}
+                         ("f32", 256, 512): (2370306304 - 1314000) / (3 * 160),
+                         ("f32", 16, 4096): 531040512 / 352,
+                         ("f64", 16, 4096): 660414720 / 176}
 
 
 def ninv_kernel(t: dict, prec: str) -> str:
@@ -875,7 +878,7 @@ def main():
                 "per_application_ms": {k: round(v, 4) for k, v in per.items()},
                 "algorithmic_bytes": ab}
     if dom == "Ninv" and ninv_tile.get("right_angle"):
-        roofline["limiter"] = ("not DRAM (the scratch of a group of tiles stays in L2): in FP32 the row kernel's "
+        roofline["limiter"] = ("not DRAM (the scratch of a group of tiles is read from L2): in FP32 the row kernel's "
                                "shared memory and instruction issue, in FP64 its load latency at 16 warps an SM (ncu)")
     elif dom == "Ninv" and ninv_tile.get("split"):
         # what the ncu captures show about the split kernels

@@ -201,6 +201,7 @@ int mdp_mem_get(size_t nbytes, void **p, size_t *got, int *dev) {
     cudaError_t e = cudaMalloc(p, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
+        mem_flush();
         mdp_mem_trim(*dev);
         e = cudaMalloc(p, want);
     }

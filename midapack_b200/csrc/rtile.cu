@@ -503,7 +503,8 @@ __global__ void __launch_bounds__(256, rt_ctas<T>()) rt_rows_kernel(RArgs<T> a) 
 // ------------------------------------------------------------------ host side
 template <typename T> size_t rows_smem(int L) { return 2 * sizeof(T) * (size_t) rt_entries(L); }
 // Items whose columns, rows and columns back are launched together, so that their scratch
-// stays in L2 (126 MB) between the three kernels.  Groups alternate between the context's
+// is read from L2 (126 MB) by the next kernel; what is written goes out to DRAM all the same (2^25
+// samples, half bandwidth 2^14, FP32: 158 MB read and 373 written, samples and outputs 134 each).  Groups alternate between the context's
 // stream and its side stream with a scratch half each: the last CTAs of one group's kernel
 // and the next launch share the device with the other group's.  64 x 2^20 samples, half
 // bandwidth 2^14, one stream and 64 MB -> two and 64 MB each: FP32 0.70 -> 0.645 ms, FP64 1.34
